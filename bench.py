@@ -430,7 +430,7 @@ def main():
     achieved = ALGO_BYTES_PER_RAY * args.rays / mean_kernel_s / 1e9
     traffic_per_ray = profiled_traffic()
 
-    fetched_per_ray = (80.0 * steps_count["node_steps"] + 48.0 * steps_count["triangle_steps"]) / args.rays
+    fetched_per_ray = (96.0 * steps_count["node_steps"] + 48.0 * steps_count["triangle_steps"]) / args.rays
     l2_achieved = fetched_per_ray * args.rays / mean_kernel_s / 1e9
 
     cpu_baseline = None
@@ -482,7 +482,7 @@ def main():
                                 "fetched_bytes_per_ray": round(fetched_per_ray, 2),
                                 "nodes_per_ray": round(steps_count["node_steps"] / args.rays, 4),
                                 "triangles_per_ray": round(steps_count["triangle_steps"] / args.rays, 4),
-                                "bytes": "80 B per 8-wide node visited + 48 B per triangle tested, "
+                                "bytes": "96 B per 8-wide node visited + 48 B per triangle tested, "
                                          "counted by spb_cast_stats_device over the same rays"}},
             "id_parity": id_parity,
             "any_hit_mrays_s": round(world * any_hit_mrays, 3),

@@ -118,7 +118,7 @@ class Tree:
 
     def traversal_stats(self, rays) -> dict:
         """Closest-hit cast of a CUDA tensor of rays that also counts the traversal's work:
-        {"rays", "node_steps", "triangle_steps"} summed over the batch (nodes visited are 80 B
+        {"rays", "node_steps", "triangle_steps"} summed over the batch (nodes visited are 96 B
         each, triangles tested 48 B each)."""
         import torch
 

@@ -477,23 +477,24 @@ bool collapse_tree(std::vector<Box> const& boxes, std::vector<float> const& cent
         Wide_node wn;
         std::memset(&wn, 0, sizeof(wn));
         for (int a = 0; a < 3; ++a) {
-            wn.origin[a]   = origin[a];
-            wn.exponent[a] = uint8_t(expo[a] + 127);
+            wn.origin[a] = origin[a];
         }
+        wn.scale_xy[0] = float(scale[0]);
+        wn.scale_xy[1] = float(scale[1]);
+        wn.scale_z     = float(scale[2]);
         wn.child_base = uint32_t(out.nodes.size());
         wn.tri_base   = uint32_t(out.triangles.size());
 
         double node_area = double(node_box.area());
         out.sah_cost += node_area / root_area;
 
-        uint32_t tri_offset = 0;
         for (int s = 0; s < 8; ++s) {
             int const c = child_in[s];
             if (c < 0) {
-                // Empty slot: inverted box, no meta bits.
+                // Empty slot: inverted box, no mask bits.
                 for (int a = 0; a < 3; ++a) {
-                    wn.qlo[a][s] = 255;
-                    wn.qhi[a][s] = 0;
+                    wn.planes[a][s][0] = 255;
+                    wn.planes[a][s][1] = 0;
                 }
                 continue;
             }
@@ -501,32 +502,30 @@ bool collapse_tree(std::vector<Box> const& boxes, std::vector<float> const& cent
             for (int a = 0; a < 3; ++a) {
                 double const lo = (double(b.box.lo[a]) - pad - double(origin[a])) / scale[a];
                 double const hi = (double(b.box.hi[a]) + pad - double(origin[a])) / scale[a];
-                wn.qlo[a][s]    = uint8_t(std::clamp(std::floor(lo), 0., 255.));
-                wn.qhi[a][s]    = uint8_t(std::clamp(std::ceil(hi), 0., 255.));
+                wn.planes[a][s][0] = uint8_t(std::clamp(std::floor(lo), 0., 255.));
+                wn.planes[a][s][1] = uint8_t(std::clamp(std::ceil(hi), 0., 255.));
             }
             if (b.count <= Max_leaf_triangles) {
                 std::vector<uint32_t> tris;
                 gather(kids[size_t(c)], tris);
                 uint32_t const cnt = uint32_t(tris.size());
-                wn.meta[s] = uint8_t((((1u << cnt) - 1u) << 5) | tri_offset);
+                wn.masks |= ((1u << cnt) - 1u) << (3 * s);
                 for (uint32_t t : tris) {
                     Wide_triangle wt;
                     std::memset(&wt, 0, sizeof(wt));
                     emit(t, wt);
                     out.triangles.push_back(wt);
                 }
-                tri_offset += cnt;
                 out.num_leaves++;
                 out.sah_cost += double(b.box.area()) / root_area * double(cnt);
             } else {
-                wn.imask |= uint8_t(1u << s);
-                wn.meta[s] = uint8_t((1u << 5) | (24u + uint32_t(s)));
+                wn.masks |= 1u << (24 + s);
             }
         }
 
         // Internal children, contiguous from child_base in slot order.
         for (int s = 0; s < 8; ++s) {
-            if (wn.imask & (1u << s)) {
+            if (wn.masks & (1u << (24 + s))) {
                 uint32_t const w = uint32_t(out.nodes.size());
                 out.nodes.emplace_back();
                 queue.push_back({w, kids[size_t(child_in[s])], job.depth + 1});

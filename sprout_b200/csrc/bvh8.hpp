@@ -1,5 +1,5 @@
 // Host-side BVH construction for the GPU cast: binned-SAH binary tree, greedy collapse to an
-// 8-wide tree, and encoding into 80-byte nodes with 8-bit quantized child boxes.
+// 8-wide tree, and encoding into 96-byte nodes with 8-bit quantized child boxes.
 #pragma once
 
 #include <cstdint>
@@ -8,41 +8,39 @@
 
 namespace spb {
 
-// One 8-wide node, 80 bytes = 5 x 16-byte words (loaded with five 128-bit loads).
-//   w0: origin.xyz (float), exponents ex|ey|ez (biased by 127, one byte each) | imask << 24
-//   w1: child_base, tri_base, meta[0..3], meta[4..7]
-//   w2: qlo_x[0..7], qlo_y[0..7]
-//   w3: qlo_z[0..7], qhi_x[0..7]
-//   w4: qhi_y[0..7], qhi_z[0..7]
-// Child slot i has the box origin + [qlo, qhi] * 2^(e - 127) per axis.  imask bit i marks an
-// internal child.  meta[i]: 0 = empty slot; internal child = 0b001 << 5 | (24 + i);
-// leaf = unary(triangle count) << 5 | offset, the leaf's triangles being
-// tri_base + offset .. tri_base + offset + count - 1 (count 1..3, offset 0..23).
-// Internal children are stored contiguously from child_base in slot order.
-struct alignas(16) Wide_node {
+// One 8-wide node, 96 bytes, loaded with three 256-bit loads.
+//   origin.xyz, tri_valid | imask << 24, child_base, tri_base, scale.x, scale.y
+//   x planes, y planes
+//   z planes, scale.z
+// Planes of an axis: byte 4 j + 2 c + s is the low (s = 0) or high (1) plane of child 2 j + c.
+// Child slot i has the box origin + [lo, hi] * scale per axis, scale a power of two.  imask bit i
+// marks an internal child; bits 3 i .. 3 i + 2 of tri_valid the triangles (1 to 3) of a leaf.  A
+// node's triangles are stored contiguously from tri_base in the order of those bits, its internal
+// children from child_base in slot order.
+struct alignas(32) Wide_node {
     float    origin[3];
-    uint8_t  exponent[3];
-    uint8_t  imask;
+    uint32_t masks;
     uint32_t child_base;
     uint32_t tri_base;
-    uint8_t  meta[8];
-    uint8_t  qlo[3][8];
-    uint8_t  qhi[3][8];
+    float    scale_xy[2];
+    uint8_t  planes[3][8][2];  // axis, child, low / high
+    float    scale_z;
+    uint32_t pad[3];
 };
-static_assert(sizeof(Wide_node) == 80, "Wide_node must be 80 bytes");
+static_assert(sizeof(Wide_node) == 96, "Wide_node must be 96 bytes");
 
-// One triangle, 48 bytes: vertex a, edges b - a and c - a (exactly the values the
+// One triangle, 64 bytes, of which 48 are read (two loads): vertex a, edges b - a and c - a (exactly the values the
 // Möller-Trumbore test computes first), the caller's triangle index and a class word the
 // traversal can filter on (the path tracer marks participating-medium boundaries).
-struct alignas(16) Wide_triangle {
+struct alignas(64) Wide_triangle {
     float    a[3];
     uint32_t id;
     float    e1[3];
     uint32_t tri_class;
     float    e2[3];
-    uint32_t pad1;
+    uint32_t pad[5];
 };
-static_assert(sizeof(Wide_triangle) == 48, "Wide_triangle must be 48 bytes");
+static_assert(sizeof(Wide_triangle) == 64, "Wide_triangle must be 64 bytes");
 
 struct Wide_bvh {
     std::vector<Wide_node>     nodes;

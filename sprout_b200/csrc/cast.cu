@@ -29,14 +29,14 @@ namespace {
 using namespace spb;
 
 // Launch shape: 128-thread blocks, registers bounded so that SPB_CAST_MIN_BLOCKS blocks fit on
-// an SM (9: 56 registers, 36 warps; measured 3 % faster than the unbounded 64 registers and
-// 6 % faster than 48 registers at 10 blocks); a warp refills once Refill_threshold of its lanes
+// an SM (8: 64 registers, 32 warps; 9 spill in the walk and are 3-12 % slower,
+// 7 are 2-7 % slower on the large batches); a warp refills once Refill_threshold of its lanes
 // are idle (8 measured best against 4, 12 and 16).
 #ifndef SPB_CAST_REFILL
 #define SPB_CAST_REFILL 8
 #endif
 #ifndef SPB_CAST_MIN_BLOCKS
-#define SPB_CAST_MIN_BLOCKS 9
+#define SPB_CAST_MIN_BLOCKS 8
 #endif
 constexpr int      Block            = 128;
 constexpr uint32_t Refill_threshold = SPB_CAST_REFILL;
@@ -55,7 +55,7 @@ constexpr uint32_t Num_counter_slots = 3;
 // into stats[0] and stats[1]); the counting variant is only launched by spb_cast_stats_device.
 template <bool Any_hit, bool Stats = false>
 __global__ void SPB_CAST_BOUNDS
-    cast_kernel(uint4 const* __restrict__ nodes, float4 const* __restrict__ triangles,
+    cast_kernel(Wide_node const* __restrict__ nodes, float4 const* __restrict__ triangles,
                 float4 const* __restrict__ rays, uint32_t num_rays, uint32_t* __restrict__ ids,
                 float* __restrict__ ts, float2* __restrict__ uvs, uint8_t* __restrict__ occluded,
                 uint32_t* __restrict__ work, uint32_t* __restrict__ overflow, float hit_margin,
@@ -66,7 +66,7 @@ __global__ void SPB_CAST_BOUNDS
     gpu::Ray_state r;
     gpu::Traversal tv;
     uint2          stack[gpu::Stack_size];
-    uint32_t       ray       = 0;
+    uint32_t       ray       = gpu::Miss;  // the lane\'s ray, until its result is written
     bool           active    = false;
     bool           exhausted = false;
     uint32_t       node_steps = 0;
@@ -114,18 +114,21 @@ __global__ void SPB_CAST_BOUNDS
             idle = __ballot_sync(Full_mask, !active);
         }
 
-        if (!active) {
-            continue;
-        }
-
-        if constexpr (Stats) {
-            if (tv.tri_group.y != 0) {
-                ++tri_steps;
-            } else if ((tv.group.y & 0xFF000000u) || tv.sp > 0) {
-                ++node_steps;
+        // The lanes walk until enough are idle for a refill, or with no rays left until all are.
+        int const floor = exhausted ? 0 : 32 - int(Refill_threshold);
+        do {
+            if constexpr (Stats) {
+                if (active) {
+                    tri_steps += tv.tri_group.y != 0;
+                    node_steps += (tv.tri_group.y & (tv.tri_group.y - 1)) == 0 &&
+                                  ((tv.group.y & 0xFF000000u) || tv.sp > 0);
+                }
             }
-        }
-        if (gpu::traversal_step<Any_hit>(r, tv, stack, nodes, triangles, hit_margin, overflow)) {
+            if (gpu::warp_step<Any_hit>(active, r, tv, stack, nodes, triangles, hit_margin, overflow)) {
+                active = false;
+            }
+        } while (__popc(__ballot_sync(Full_mask, active)) > floor);
+        if (!active && ray != gpu::Miss) {
             if (Any_hit) {
                 __stcs(occluded + ray, uint8_t(r.best_id != gpu::Miss ? 1 : 0));
             } else {
@@ -135,7 +138,7 @@ __global__ void SPB_CAST_BOUNDS
                     __stcs(uvs + ray, make_float2(r.u, r.v));
                 }
             }
-            active = false;
+            ray = gpu::Miss;
         }
     }
     if constexpr (Stats) {
@@ -171,7 +174,7 @@ struct spb_tree {
     int           num_sms    = 0;
     int           grid_hit   = 0;
     int           grid_any   = 0;
-    uint4*        d_nodes    = nullptr;
+    spb::Wide_node* d_nodes  = nullptr;
     float4*       d_tris     = nullptr;
     uint32_t*     d_counters = nullptr;
     unsigned long long* d_stats = nullptr;  // node steps, triangle steps (spb_cast_stats_device)
@@ -258,11 +261,11 @@ int32_t launch(spb_tree* tree, bool any_hit, uint32_t slot, float4 const* rays, 
     int const grid = std::max(1, std::min(full, need));
     if (any_hit) {
         cast_kernel<true><<<grid, Block, 0, stream>>>(
-            reinterpret_cast<uint4 const*>(tree->d_nodes), tree->d_tris, rays, n, nullptr,
+            tree->d_nodes, tree->d_tris, rays, n, nullptr,
             nullptr, nullptr, occ, counters, counters + 1, tree->hit_margin, tree->scene_lo, tree->scene_hi, nullptr);
     } else {
         cast_kernel<false><<<grid, Block, 0, stream>>>(
-            reinterpret_cast<uint4 const*>(tree->d_nodes), tree->d_tris, rays, n, ids, ts, uvs,
+            tree->d_nodes, tree->d_tris, rays, n, ids, ts, uvs,
             nullptr, counters, counters + 1, tree->hit_margin, tree->scene_lo, tree->scene_hi, nullptr);
     }
     SPB_CUDA(cudaGetLastError());
@@ -473,7 +476,7 @@ extern "C" SPB_API int32_t spb_cast_stats_device(spb_tree* tree, float const* ra
     uint32_t const n    = uint32_t(num_rays);
     int const      grid = std::max(1, std::min(tree->grid_hit, int((uint64_t(n) + Block - 1) / Block)));
     cast_kernel<false, true><<<grid, Block, 0, st>>>(
-        reinterpret_cast<uint4 const*>(tree->d_nodes), tree->d_tris,
+        tree->d_nodes, tree->d_tris,
         reinterpret_cast<float4 const*>(rays), n, ids, ts, nullptr, nullptr, counters,
         counters + 1, tree->hit_margin, tree->scene_lo, tree->scene_hi, tree->d_stats);
     SPB_CUDA(cudaGetLastError());
@@ -681,7 +684,7 @@ extern "C" SPB_API int32_t spb_intersect_host_static(spb_tree* tree, float const
     SPB_CUDA(cudaMemsetAsync(work, 0, sizeof(uint32_t), nullptr));
     SPB_CUDA(cudaMemcpyAsync(d_rays, rays, size_t(n) * 32, cudaMemcpyHostToDevice, nullptr));
     int const grid = std::max(1, std::min(tree->grid_hit, int((n + Block - 1) / Block)));
-    cast_kernel<false><<<grid, Block, 0, nullptr>>>(reinterpret_cast<uint4 const*>(tree->d_nodes),
+    cast_kernel<false><<<grid, Block, 0, nullptr>>>(tree->d_nodes,
                                                     tree->d_tris, d_rays, n, d_ids, d_ts, nullptr,
                                                     nullptr, work, tree->d_counters + 1,
                                                     tree->hit_margin, tree->scene_lo, tree->scene_hi, nullptr);

@@ -146,7 +146,7 @@ struct Emission_dist_gpu {
 };
 
 struct Scene_gpu {
-    uint4 const*              nodes;
+    Wide_node const*          nodes;
     float4 const*             tris;
     float                     hit_margin;
     uint4 const*              tri_info;  // v0, v1, v2, material
@@ -630,7 +630,7 @@ __global__ void __launch_bounds__(Trace_block)
     gpu::Traversal      tv;
     gpu::Instance_state is;
     uint2               stack[gpu::Stack_size];
-    uint32_t       path      = 0;
+    uint32_t       path      = gpu::Miss;  // the lane's entry, until its result is written
     bool           active    = false;
     bool           exhausted = false;
 
@@ -675,12 +675,15 @@ __global__ void __launch_bounds__(Trace_block)
                 }
             }
         }
-        if (!active) {
-            continue;
-        }
-        if (gpu::traversal_step<Any_hit, Media, Instances>(r, tv, stack, s.nodes, s.tris, s.hit_margin,
-                                                            overflow, Class_boundary, &is,
-                                                            s.inst_trace)) {
+        // The lanes walk until enough are idle for a refill, or with no entries left until all are.
+        int const floor = exhausted ? 0 : 32 - int(Refill_threshold);
+        do {
+            if (gpu::warp_step<Any_hit, Media, Instances>(active, r, tv, stack, s.nodes, s.tris, s.hit_margin,
+                                                           overflow, Class_boundary, &is, s.inst_trace)) {
+                active = false;
+            }
+        } while (__popc(__ballot_sync(Full_mask, active)) > floor);
+        if (!active && path != gpu::Miss) {
             if (Any_hit) {
                 uint32_t const e = path & Entry_index;
                 if (r.best_id == gpu::Miss) {
@@ -721,7 +724,7 @@ __global__ void __launch_bounds__(Trace_block)
                     p.hit_inst[path] = is.best_inst;
                 }
             }
-            active = false;
+            path = gpu::Miss;
         }
     }
 }
@@ -3332,7 +3335,7 @@ __global__ void k_resolve(float4 const* film, float4 const* comp, uint32_t n, fl
 
 struct Renderer::Device {
     // scene
-    uint4*             nodes      = nullptr;
+    Wide_node*         nodes      = nullptr;
     float4*            tris       = nullptr;
     uint4*             tri_info   = nullptr;
     float4*            positions  = nullptr;
