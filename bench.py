@@ -489,7 +489,8 @@ def main():
             "render": render,
             "e2e": e2e,
             "cpu_baseline": cpu_baseline,
-            "gpu_launches": args.steps,
+            # from 2^20 rays on, a cast chooses between two forms of its kernel: three launches
+            "gpu_launches": args.steps * (3 if args.rays >= 1 << 20 else 1),
             "clocks": clocks.summary(),
         }
         print(json.dumps(line))

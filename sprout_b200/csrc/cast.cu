@@ -1,16 +1,29 @@
 // GPU ray cast: closest hit and any hit over the 8-wide quantized BVH built in bvh8.cpp.
 //
 // Kernel design (sm_100a):
-//  * Persistent warps with dynamic ray fetch: each warp keeps 32 rays in flight; whenever
-//    at least Refill_threshold lanes have finished, the warp takes that many new ray indices
-//    with one atomicAdd on the launch's work counter, so lanes stay busy although ray costs
-//    differ by orders of magnitude.
+//  * Persistent warps with dynamic ray fetch: each warp keeps 32 rays in flight.  Its lanes walk
+//    together (gpu::warp_step) until Refill_threshold of them have finished; those answer their
+//    rays and fetch new ones, so lanes stay busy although ray costs differ by orders of magnitude.
 //  * A fetched ray is first tested against the tree's padded scene box (gpu::enters_box, in
-//    double precision); one that misses it (72 % of the benchmark's rays) is answered as a
-//    miss at once, without the 8-child test of the root node.
+//    double precision); one that misses it is answered at once, without the 8-child test of the
+//    root node.  Where most rays miss it, a second form of the kernel fetches and tests 64 rays
+//    at a time with all lanes (choose_kernel).
+//  * A batch with at most a ray for each resident lane is dealt out in fixed shares of 32 rays a
+//    warp: no work counter, so no memset before the kernel.
 //  * Rays are loaded with evict-first hints and results stored with streaming stores, so the
-//    512 MiB of benchmark rays do not push the tree (63 MiB) out of L2.
+//    512 MiB of benchmark rays do not push the tree (83 MB) out of L2.
 //  * Traversal, triangle test and hit definition: traverse.cuh.
+//
+// What bounds it, and what it measured (B200; before: every lane stepping by itself through
+// 80-byte nodes, one launch form): the start's kernel kept 9.8 of 32 lanes busy and its ALU pipe
+// 70 % (29 warp instructions a step); now 19.4 lanes and 12, and what is left is the latency of
+// dependent node loads (32 warps an SM) and L1's one tag look-up a cycle for each lane's line.
+//   16,777,216 incoherent closest-hit rays, 1,048,576 triangles: 2,540 -> 1,205 us
+//   4,194,301 short any-hit rays from its surface: 2,600 -> 1,265 us
+//   360,000 primary rays, 65,536 triangles: 253 -> 125 us; 4,099 any-hit rays: 37 -> 23 us
+// Tried and not kept: ray batches copied to shared memory ahead of use (cp.async, one batch ahead:
+// 1,250, 1,360 and 170 us on the first three, for claimed batches wait while other warps run dry);
+// the closest hit's barycentrics recomputed at the end instead of carried (1 % slower).
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -19,6 +32,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 
 #include "bvh8.hpp"
 #include "common.hpp"
@@ -29,9 +43,9 @@ namespace {
 using namespace spb;
 
 // Launch shape: 128-thread blocks, registers bounded so that SPB_CAST_MIN_BLOCKS blocks fit on
-// an SM (8: 64 registers, 32 warps; 9 spill in the walk and are 3-12 % slower,
-// 7 are 2-7 % slower on the large batches); a warp refills once Refill_threshold of its lanes
-// are idle (8 measured best against 4, 12 and 16).
+// an SM (8: 64 registers, 32 warps; 9 spill in the walk and are 3-12 % slower, 7 are 2-7 % slower
+// on the large batches); a warp refills once Refill_threshold of its lanes are idle (4 and 12 are
+// 1-4 % slower).
 #ifndef SPB_CAST_REFILL
 #define SPB_CAST_REFILL 8
 #endif
@@ -46,76 +60,171 @@ constexpr uint32_t Refill_threshold = SPB_CAST_REFILL;
 #define SPB_CAST_BOUNDS __launch_bounds__(Block)
 #endif
 constexpr uint32_t Full_mask        = 0xFFFFFFFFu;
+constexpr uint32_t Waiting          = 64;  // rays a warp of the sparse form fetches together
 
 // Counter slots (2 words each: work counter, overflow count).  Slot 0 serves the device
 // entry points, slots 1 and 2 the two streams of the host pipeline.
 constexpr uint32_t Num_counter_slots = 3;
+// After them, one word a slot: the form of kernel its cast takes (choose_kernel).
+constexpr uint32_t Num_counter_words = 3 * Num_counter_slots;
+
+// From this many rays on, a cast chooses between the two forms of the kernel.  The choice costs
+// two launches (about 8 us); at 2^20 rays a cast takes 70 us or more, and the sparse form saves a
+// quarter where it is the better one.
+constexpr uint32_t Choose_rays = 1u << 20;
+constexpr uint32_t Probes      = 256;
+
+// Answers a ray that misses the scene box.
+template <bool Any_hit>
+__device__ __forceinline__ void answer_miss(uint32_t i, float t, uint32_t* ids, float* ts, float2* uvs,
+                                            uint8_t* occluded) {
+    if (Any_hit) {
+        __stcs(occluded + i, uint8_t(0));
+    } else {
+        __stcs(ids + i, gpu::Miss);
+        __stcs(ts + i, t);
+        if (uvs) {
+            __stcs(uvs + i, make_float2(0.f, 0.f));
+        }
+    }
+}
+
+// Chooses the form of a large cast: *sparse = 1 if most of Probes rays spread over the batch miss
+// the scene box.  One block of Probes threads.  (The sparse form: 16,777,216 rays of which 28 %
+// enter, 1,205 against 1,566 us; 4,194,301 rays that all enter, 1,320 against 1,265 us, because
+// its queue takes registers from the walk.)
+__global__ void choose_kernel(float4 const* __restrict__ rays, uint32_t num_rays, float3 scene_lo, float3 scene_hi,
+                              uint32_t* __restrict__ sparse) {
+    uint32_t const i = uint32_t(uint64_t(threadIdx.x) * num_rays / Probes);
+    gpu::Ray_state r;
+    gpu::Traversal tv;
+    gpu::start_ray(r, tv, __ldg(rays + 2 * size_t(i)), __ldg(rays + 2 * size_t(i) + 1));
+    int const entering = __syncthreads_count(gpu::enters_box(r, scene_lo, scene_hi));
+    if (threadIdx.x == 0) {
+        *sparse = 2 * entering < int(Probes) ? 1u : 0u;
+    }
+}
+
+// Waiting rays from index base on, two a lane: those that enter the scene box are put into the
+// warp's queue, the others answered.  Returns how many entered.  Out of line: its registers must
+// not add to those of the walk.
+template <bool Any_hit>
+__device__ __noinline__ uint32_t fetch_sparse(float4 const* rays, uint32_t base, uint32_t num_rays, float3 scene_lo,
+                                              float3 scene_hi, uint32_t* queue, uint32_t* ids, float* ts,
+                                              float2* uvs, uint8_t* occluded) {
+    constexpr uint32_t Each   = Waiting / 32;
+    uint32_t const     lane   = threadIdx.x & 31u;
+    uint32_t           queued = 0;
+    float4             o[Each], d[Each];
+#pragma unroll
+    for (uint32_t h = 0; h < Each; ++h) {
+        size_t const i = min(base + 32 * h + lane, num_rays - 1);
+        o[h]           = __ldcs(rays + 2 * i);
+        d[h]           = __ldcs(rays + 2 * i + 1);
+    }
+#pragma unroll
+    for (uint32_t h = 0; h < Each; ++h) {
+        uint32_t const i     = base + 32 * h + lane;
+        bool           enter = false;
+        if (i < num_rays) {
+            gpu::Ray_state r;
+            gpu::Traversal tv;
+            gpu::start_ray(r, tv, o[h], d[h]);
+            enter = gpu::enters_box(r, scene_lo, scene_hi);
+            if (!enter) {
+                answer_miss<Any_hit>(i, r.tbest, ids, ts, uvs, occluded);
+            }
+        }
+        uint32_t const mask = __ballot_sync(Full_mask, enter);
+        if (enter) {
+            queue[queued + __popc(mask & ((1u << lane) - 1u))] = i;
+        }
+        queued += __popc(mask);
+    }
+    __syncwarp();
+    return queued;
+}
 
 // Stats: also count, per ray, the node and triangle steps of its traversal (summed per warp
 // into stats[0] and stats[1]); the counting variant is only launched by spb_cast_stats_device.
-template <bool Any_hit, bool Stats = false>
+// work: the work counter, or null for fixed shares.  form (may be null): the form chosen for the
+// cast; the other one has nothing to do.
+template <bool Any_hit, bool Sparse, bool Stats = false>
 __global__ void SPB_CAST_BOUNDS
     cast_kernel(Wide_node const* __restrict__ nodes, float4 const* __restrict__ triangles,
                 float4 const* __restrict__ rays, uint32_t num_rays, uint32_t* __restrict__ ids,
                 float* __restrict__ ts, float2* __restrict__ uvs, uint8_t* __restrict__ occluded,
-                uint32_t* __restrict__ work, uint32_t* __restrict__ overflow, float hit_margin,
+                uint32_t* __restrict__ work, uint32_t const* __restrict__ form,
+                uint32_t* __restrict__ overflow, float hit_margin,
                 float3 scene_lo, float3 scene_hi, unsigned long long* __restrict__ stats) {
+    if (form && (*form != 0) != Sparse) {
+        return;
+    }
     uint32_t const lane = threadIdx.x & 31u;
     uint32_t const lt   = (1u << lane) - 1u;
 
     gpu::Ray_state r;
     gpu::Traversal tv;
     uint2          stack[gpu::Stack_size];
-    uint32_t       ray       = gpu::Miss;  // the lane\'s ray, until its result is written
+    uint32_t       ray       = gpu::Miss;  // the lane's ray, until its result is written
     bool           active    = false;
     bool           exhausted = false;
     uint32_t       node_steps = 0;
     uint32_t       tri_steps  = 0;
 
-    while (true) {
-        uint32_t idle = __ballot_sync(Full_mask, !active);
-        if (exhausted && idle == Full_mask) {
-            break;
-        }
-        // Refill while enough lanes are idle.  A fetched ray that misses the scene box is
-        // answered at once (a miss) and its lane stays idle for the next round of the loop.
-        while (!exhausted && __popc(idle) >= int(Refill_threshold)) {
-            uint32_t const count  = __popc(idle);
-            uint32_t const leader = __ffs(idle) - 1;
-            uint32_t       base   = 0;
-            if (lane == leader) {
+    // Takes `count` ray indices for the warp.
+    auto const take = [&](uint32_t count) {
+        uint32_t base = (blockIdx.x * (Block / 32) + threadIdx.x / 32) * 32u;
+        if (work) {
+            if (lane == 0) {
                 base = atomicAdd(work, count);
             }
-            base = __shfl_sync(Full_mask, base, leader);
-            if (uint64_t(base) + count >= num_rays) {
-                exhausted = true;
-            }
-            if (!active) {
-                uint32_t const mine = base + __popc(idle & lt);
-                if (mine < num_rays) {
-                    // Rays are read once: evict-first loads keep them from displacing the
-                    // tree's nodes and triangles in L2.
-                    gpu::start_ray(r, tv, __ldcs(rays + 2 * size_t(mine)),
-                                   __ldcs(rays + 2 * size_t(mine) + 1));
-                    if (gpu::enters_box(r, scene_lo, scene_hi)) {
-                        ray    = mine;
-                        active = true;
-                    } else if (Any_hit) {
-                        __stcs(occluded + mine, uint8_t(0));
+            base = __shfl_sync(Full_mask, base, 0);
+        }
+        exhausted = !work || uint64_t(base) + count >= num_rays;
+        return base;
+    };
+
+    __shared__ uint32_t waiting[Sparse ? Block / 32 : 1][Waiting];
+    uint32_t            queued = 0;  // Sparse: the warp's fetched rays that wait for a lane
+    while (true) {
+        uint32_t idle = __ballot_sync(Full_mask, !active);
+        while ((!exhausted || queued != 0) && __popc(idle) >= int(Refill_threshold)) {
+            uint32_t const want = __popc(idle);
+            if constexpr (Sparse) {
+                uint32_t const  rank  = __popc(idle & lt);
+                uint32_t* const queue = waiting[threadIdx.x / 32];
+                if (queued == 0) {
+                    queued = fetch_sparse<Any_hit>(rays, take(Waiting), num_rays, scene_lo, scene_hi, queue, ids, ts,
+                                                   uvs, occluded);
+                }
+                uint32_t const given = min(queued, want);
+                if (!active && rank < given) {
+                    ray = queue[queued - 1u - rank];
+                    gpu::start_ray(r, tv, __ldcs(rays + 2 * size_t(ray)), __ldcs(rays + 2 * size_t(ray) + 1));
+                    active = true;
+                }
+                queued -= given;
+                __syncwarp();
+            } else {
+                uint32_t const i = take(want) + __popc(idle & lt);
+                if (!active && i < num_rays) {
+                    gpu::start_ray(r, tv, __ldcs(rays + 2 * size_t(i)), __ldcs(rays + 2 * size_t(i) + 1));
+                    active = gpu::enters_box(r, scene_lo, scene_hi);
+                    if (active) {
+                        ray = i;
                     } else {
-                        __stcs(ids + mine, gpu::Miss);
-                        __stcs(ts + mine, r.tbest);
-                        if (uvs) {
-                            __stcs(uvs + mine, make_float2(0.f, 0.f));
-                        }
+                        answer_miss<Any_hit>(i, r.tbest, ids, ts, uvs, occluded);
                     }
                 }
             }
             idle = __ballot_sync(Full_mask, !active);
         }
-
+        if (idle == Full_mask) {
+            break;
+        }
         // The lanes walk until enough are idle for a refill, or with no rays left until all are.
-        int const floor = exhausted ? 0 : 32 - int(Refill_threshold);
+        int const floor = exhausted && queued == 0 ? 0 : 32 - int(Refill_threshold);
         do {
             if constexpr (Stats) {
                 if (active) {
@@ -252,22 +361,36 @@ int32_t ensure_pipeline(spb_tree* tree) {
     return SPB_OK;
 }
 
+// Blocks of a cast of n rays, of at most `full`.  With a ray or less for each of their lanes the
+// warps take fixed shares of 32 rays (fixed), otherwise they take rays from the work counter.
+int launch_shape(uint32_t n, int full, bool& fixed) {
+    uint64_t const need = (uint64_t(n) + Block - 1) / Block;
+    fixed               = need <= uint64_t(full);
+    return fixed ? int(need) : full;
+}
+
 int32_t launch(spb_tree* tree, bool any_hit, uint32_t slot, float4 const* rays, uint32_t n,
                uint32_t* ids, float* ts, float2* uvs, uint8_t* occ, cudaStream_t stream) {
-    uint32_t* counters = tree->d_counters + 2 * slot;
-    SPB_CUDA(cudaMemsetAsync(counters, 0, sizeof(uint32_t), stream));
-    int const full = any_hit ? tree->grid_any : tree->grid_hit;
-    int const need = int((uint64_t(n) + Block - 1) / Block);
-    int const grid = std::max(1, std::min(full, need));
-    if (any_hit) {
-        cast_kernel<true><<<grid, Block, 0, stream>>>(
-            tree->d_nodes, tree->d_tris, rays, n, nullptr,
-            nullptr, nullptr, occ, counters, counters + 1, tree->hit_margin, tree->scene_lo, tree->scene_hi, nullptr);
-    } else {
-        cast_kernel<false><<<grid, Block, 0, stream>>>(
-            tree->d_nodes, tree->d_tris, rays, n, ids, ts, uvs,
-            nullptr, counters, counters + 1, tree->hit_margin, tree->scene_lo, tree->scene_hi, nullptr);
+    uint32_t* const counters = tree->d_counters + 2 * slot;
+    bool            fixed    = false;
+    int const       grid     = launch_shape(n, any_hit ? tree->grid_any : tree->grid_hit, fixed);
+    uint32_t* const work     = fixed ? nullptr : counters;
+    if (work) {
+        SPB_CUDA(cudaMemsetAsync(work, 0, sizeof(uint32_t), stream));
     }
+    auto const cast = [&](auto Any_hit, auto Sparse, uint32_t const* form) {
+        cast_kernel<decltype(Any_hit)::value, decltype(Sparse)::value><<<grid, Block, 0, stream>>>(
+            tree->d_nodes, tree->d_tris, rays, n, ids, ts, uvs, occ, work, form, counters + 1, tree->hit_margin,
+            tree->scene_lo, tree->scene_hi, nullptr);
+    };
+    uint32_t const* form = nullptr;
+    if (n >= Choose_rays) {
+        uint32_t* const chosen = tree->d_counters + 2 * Num_counter_slots + slot;
+        choose_kernel<<<1, Probes, 0, stream>>>(rays, n, tree->scene_lo, tree->scene_hi, chosen);
+        form = chosen;
+        any_hit ? cast(std::true_type(), std::true_type(), form) : cast(std::false_type(), std::true_type(), form);
+    }
+    any_hit ? cast(std::true_type(), std::false_type(), form) : cast(std::false_type(), std::false_type(), form);
     SPB_CUDA(cudaGetLastError());
     return SPB_OK;
 }
@@ -296,18 +419,18 @@ extern "C" SPB_API int32_t spb_tree_create(spb_tree** out) {
     int per_sm_hit = 0;
     int per_sm_any = 0;
     if (e == cudaSuccess) {
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_hit, cast_kernel<false>, Block,
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_hit, cast_kernel<false, false>, Block,
                                                           0);
     }
     if (e == cudaSuccess) {
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_any, cast_kernel<true>, Block,
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_any, cast_kernel<true, false>, Block,
                                                           0);
     }
     if (e == cudaSuccess) {
-        e = cudaMalloc(&tree->d_counters, 2 * Num_counter_slots * sizeof(uint32_t));
+        e = cudaMalloc(&tree->d_counters, Num_counter_words * sizeof(uint32_t));
     }
     if (e == cudaSuccess) {
-        e = cudaMemset(tree->d_counters, 0, 2 * Num_counter_slots * sizeof(uint32_t));
+        e = cudaMemset(tree->d_counters, 0, Num_counter_words * sizeof(uint32_t));
     }
     if (e == cudaSuccess) {
         e = cudaMalloc(&tree->d_stats, 2 * sizeof(unsigned long long));
@@ -475,9 +598,9 @@ extern "C" SPB_API int32_t spb_cast_stats_device(spb_tree* tree, float const* ra
     SPB_CUDA(cudaMemsetAsync(tree->d_stats, 0, 2 * sizeof(unsigned long long), st));
     uint32_t const n    = uint32_t(num_rays);
     int const      grid = std::max(1, std::min(tree->grid_hit, int((uint64_t(n) + Block - 1) / Block)));
-    cast_kernel<false, true><<<grid, Block, 0, st>>>(
+    cast_kernel<false, false, true><<<grid, Block, 0, st>>>(
         tree->d_nodes, tree->d_tris,
-        reinterpret_cast<float4 const*>(rays), n, ids, ts, nullptr, nullptr, counters,
+        reinterpret_cast<float4 const*>(rays), n, ids, ts, nullptr, nullptr, counters, nullptr,
         counters + 1, tree->hit_margin, tree->scene_lo, tree->scene_hi, tree->d_stats);
     SPB_CUDA(cudaGetLastError());
     unsigned long long host[2] = {0, 0};
@@ -681,12 +804,15 @@ extern "C" SPB_API int32_t spb_intersect_host_static(spb_tree* tree, float const
     // The array keeps the previous call's contents: the work counter must start at zero.
     // Stack overflows (none for trees this library builds) are counted in the tree's own
     // counter, as spb_intersect_host counts them, and reported by spb_tree_status.
-    SPB_CUDA(cudaMemsetAsync(work, 0, sizeof(uint32_t), nullptr));
+    bool      fixed = false;
+    int const grid  = launch_shape(n, tree->grid_hit, fixed);
+    if (!fixed) {
+        SPB_CUDA(cudaMemsetAsync(work, 0, sizeof(uint32_t), nullptr));
+    }
     SPB_CUDA(cudaMemcpyAsync(d_rays, rays, size_t(n) * 32, cudaMemcpyHostToDevice, nullptr));
-    int const grid = std::max(1, std::min(tree->grid_hit, int((n + Block - 1) / Block)));
-    cast_kernel<false><<<grid, Block, 0, nullptr>>>(tree->d_nodes,
+    cast_kernel<false, false><<<grid, Block, 0, nullptr>>>(tree->d_nodes,
                                                     tree->d_tris, d_rays, n, d_ids, d_ts, nullptr,
-                                                    nullptr, work, tree->d_counters + 1,
+                                                    nullptr, fixed ? nullptr : work, nullptr, tree->d_counters + 1,
                                                     tree->hit_margin, tree->scene_lo, tree->scene_hi, nullptr);
     SPB_CUDA(cudaGetLastError());
     SPB_CUDA(cudaMemcpyAsync(ids, d_ids, size_t(n) * 4, cudaMemcpyDeviceToHost, nullptr));

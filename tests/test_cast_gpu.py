@@ -215,3 +215,35 @@ def test_degenerate_and_clustered_triangles():
         occ = tree.intersect_p(rays)
     assert_exact(ids, t, want)
     assert np.array_equal(occ, want["occluded"])
+
+
+# Sizes about the kernel's rules: a warp's and a block's share, as many rays as lanes are resident
+# (fixed shares up to there), and the size from which a cast chooses between its two forms.
+RULE_SIZES = [1, 31, 33, 127, 129, 4099, 148 * 8 * 128, 148 * 8 * 128 + 1, (1 << 20) - 1, (1 << 20) + 33]
+
+
+@pytest.mark.parametrize("extent", [0.5, 6.0], ids=["most_enter", "most_miss"])
+@pytest.mark.parametrize("count", RULE_SIZES)
+def test_every_launch_rule_bit_exact(torch_cuda, count, extent):
+    """Both forms of the kernel and both ways of dealing out rays, against the restatement; among
+    the rays axis-parallel, zero and NaN directions and odd [min_t, max_t]."""
+    torch = torch_cuda
+    pos, idx = oracle.synth_sphere_mesh(8, 0.1, 1)
+    rays = oracle.synth_rays(count, 5, extent=extent)
+    rays[3::101, 4:7] = [0.0, 0.0, 1.0]
+    rays[5::101, 4:7] = [-1.0, 0.0, -0.0]
+    rays[7::101, 4:7] = 0.0
+    rays[9::101, 4:7] = np.nan
+    rays[11::101, 3] = -3.0
+    rays[13::101, 7] = np.inf
+    rays[15::101, 3], rays[15::101, 7] = 2.0, 1.0
+    want = oracle.restated_cast(pos, idx, rays)
+    with sb.Tree() as tree:
+        tree.build(pos, idx)
+        ids, t, uv = tree.intersect(torch.from_numpy(rays).cuda(), want_uv=True)
+        occ = tree.intersect_p(torch.from_numpy(rays).cuda())
+        assert tree.status() == 0
+    assert_exact(ids.cpu().numpy().view(np.uint32), t.cpu().numpy(), want)
+    hit = want["ids"] != MISS
+    assert np.array_equal(_bits(uv.cpu().numpy()[hit]), _bits(want["uv"][hit]))
+    assert np.array_equal(occ.cpu().numpy(), want["occluded"])
