@@ -65,6 +65,11 @@ SPB_HD V3 operator/(V3 a, float s) {
 SPB_HD float dot(V3 a, V3 b) {
     return a.x * b.x + a.y * b.y + a.z * b.z;
 }
+// dot with its roundings fixed (the compiler's choice of the inner FMA depends on the code around
+// it): where code that is compiled more than once must agree.
+SPB_HD float dot_fixed(V3 a, V3 b) {
+    return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x));
+}
 SPB_HD V3 cross(V3 a, V3 b) {
     return v3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
 }
@@ -351,13 +356,17 @@ SPB_HD bool same_hemisphere(Context const& c, V3 v) {
 }
 
 // Substitute::evaluate (substitute_sample.cpp:10-24).
+// Fixed: with the roundings of the two products below that the compiler chose differently when
+// the code around an inlined copy changed (dot_fixed).
+template <bool Fixed = false>
 SPB_HD Bxdf substitute_evaluate(Material const& m, float const* e_table, Context const& c, V3 wi) {
     if (!same_hemisphere(c, c.wo)) {
         return Bxdf{v3(0.f, 0.f, 0.f), 0.f};
     }
-    V3 const    h        = normalize(c.wo + wi);
+    V3 const    wh       = c.wo + wi;
+    V3 const    h        = Fixed ? (1.f / std::sqrt(dot_fixed(wh, wh))) * wh : normalize(wh);
     float const wo_dot_h = clamp_dot(c.wo, h);
-    float const n_dot_wi = clamp_dot(c.frame.n, wi);
+    float const n_dot_wi = Fixed ? clampf(dot_fixed(c.frame.n, wi), Dot_min, 1.f) : clamp_dot(c.frame.n, wi);
     float const n_dot_wo = clamp_abs_dot(c.frame.n, c.wo);
     float const n_dot_h  = saturate(dot(c.frame.n, h));
 

@@ -55,6 +55,7 @@ __device__ __forceinline__ V3 f3v(float4 a) {
 constexpr uint32_t Full_mask        = 0xFFFFFFFFu;
 constexpr int      Trace_block      = 128;
 constexpr int      Shade_block      = 256;
+
 constexpr uint32_t Refill_threshold = 8;
 constexpr float    Ray_max_t        = 3.4027715434167032e+38f;
 constexpr int      Filter_samples   = 30;
@@ -617,8 +618,10 @@ struct Transmit_out {
 // medium boundaries and unoccluded ones go to the transmittance queue instead of adding
 // their contribution directly.
 // Instances: the scene is a top-level tree over instances of per-mesh trees.
+// Registers for 8 blocks on an SM (64), 7 with instances (72): the walk waits on node loads, so
+// warps count; unbounded it takes 72 and 81.
 template <bool Any_hit, bool Media = false, bool Instances = false>
-__global__ void __launch_bounds__(Trace_block)
+__global__ void __launch_bounds__(Trace_block, Instances ? 7 : 8)
     k_trace(Scene_gpu s, Paths p, uint32_t const* __restrict__ queue,
             uint32_t const* __restrict__ count, uint32_t* fetch, uint32_t* overflow,
             Transmit_out tq = Transmit_out{}) {
@@ -1116,6 +1119,8 @@ __device__ bool sample_volume_light(Scene_gpu const& s, uint32_t index, V3 ps, V
     return true;
 }
 
+// Media: the scene may have volume lights.
+template <bool Media = true>
 __device__ __forceinline__ bool sample_light(Scene_gpu const& s, V3 ps, V3 n, bool total_sphere,
                                              Light_pick pk, float r1, float r2, Rng& rng, Light_sample& ls) {
     if (pk.light == Env_pick) {
@@ -1137,7 +1142,7 @@ __device__ __forceinline__ bool sample_light(Scene_gpu const& s, V3 ps, V3 n, bo
     }
     uint32_t const l       = pk.light;
     float4 const   la      = s.light_tris[3 * l + 0];
-    if (la.w < 0.f) {
+    if (Media && la.w < 0.f) {
         return sample_volume_light(s, uint32_t(-1.f - la.w), ps, n, total_sphere, pk.pdf, r1, r2, rng.uniform(),
                                    ls);
     }
@@ -1757,6 +1762,17 @@ struct Shade_out {
     uint32_t* count_records;  // split records
 };
 
+// The k-th light of a selection; out of line, as only selections of more than two walk again.
+__device__ __noinline__ Light_pick light_at(Scene_gpu const& s, V3 p, V3 n, bool total_sphere, float r, bool split,
+                                            uint32_t k) {
+    Light_pick got = {0u, 0.f};
+    walk_lights(s, p, n, total_sphere, r, split, [&](uint32_t i, Light_pick pk) {
+        got = pk;
+        return i < k;
+    });
+    return got;
+}
+
 // Next-event estimation at a vertex (sample_lights / evaluate_light, pathtracer_mis.cpp:281-347):
 // the lights select_lights chooses with the random number `select`, a sample on each (the
 // pixel's golden ratio dimension of that light at the first vertices, else the path's random
@@ -1764,7 +1780,7 @@ struct Shade_out {
 // first light) takes the path's second shadow slot; a single other light the first slot;
 // several emitters get a split record and a pick each, their contributions summed by
 // k_pick_sum after the shadow rays.  shadow / shadow2: the slots hold rays.
-template <class Eval>
+template <bool Media, bool Guided, class Eval>
 __device__ __forceinline__ void next_event(Scene_gpu const& s, Paths const& p, Wave const& wave,
                                            Shade_out const& out, uint32_t path, V3 ps, V3 n,
                                            bool total_sphere, uint32_t depth, float select, Rng& rng,
@@ -1782,18 +1798,7 @@ __device__ __forceinline__ void next_event(Scene_gpu const& s, Paths const& p, W
         }
         return true;
     });
-    auto const pick_at = [&](uint32_t k) {
-        if (k < 2) {
-            return k == 0 ? first0 : first1;
-        }
-        Light_pick got = {0u, 0.f};
-        walk_lights(s, ps, n, total_sphere, select, split, [&](uint32_t i, Light_pick pk) {
-            got = pk;
-            return i < k;
-        });
-        return got;
-    };
-    auto const     point = [&](uint32_t l, float& r1, float& r2) {
+    auto const point = [&](uint32_t l, float& r1, float& r2) {
         if (golden) {
             float2 const g = golden_2d(wave, gpixel, gsample, golden_light_2d(depth, l));
             r1             = g.x;
@@ -1803,52 +1808,107 @@ __device__ __forceinline__ void next_event(Scene_gpu const& s, Paths const& p, W
             r2 = rng.uniform();
         }
     };
-    auto const slot = [&](uint32_t l, bool second) {
-        float r1, r2;
-        point(l, r1, r2);
-        Light_sample ls;
-        if (sample_light(s, ps, n, total_sphere, pick_at(l), r1, r2, rng, ls)) {
-            V3 const c = eval(ls);
-            if (shading::max_component(c) > 0.f) {
-                store_shadow(p, path, second, ps, ls, c, depth);
-                return true;
+    if constexpr (Guided) {
+        // Slots and picks apart, as the guide was trained with: its online training amplifies the
+        // last bit of every contribution, and the loop below rounds a few of them differently.
+        auto const pick_at = [&](uint32_t k) {
+            return k == 0 ? first0 : k == 1 ? first1 : light_at(s, ps, n, total_sphere, select, split, k);
+        };
+        auto const slot = [&](uint32_t l, bool second) {
+            float r1, r2;
+            point(l, r1, r2);
+            Light_sample ls;
+            if (sample_light<Media>(s, ps, n, total_sphere, pick_at(l), r1, r2, rng, ls)) {
+                V3 const c = eval(ls);
+                if (shading::max_component(c) > 0.f) {
+                    store_shadow(p, path, second, ps, ls, c, depth);
+                    return true;
+                }
+            }
+            return false;
+        };
+        uint32_t first = 0;
+        if (m > 1 && first0.light == Env_pick) {
+            shadow2 = slot(0, true);
+            first   = 1;
+        }
+        uint32_t const count = m - first;
+        if (count == 1) {
+            shadow = slot(first, false);
+        }
+        if (count < 2) {
+            return;
+        }
+        uint32_t const base = atomicAdd(out.count_picks, count);
+        uint32_t const rec  = atomicAdd(out.count_records, 1u);
+        p.split_o[rec]      = make_float4(ps.x, ps.y, ps.z, __uint_as_float(path));
+        p.split_m[rec]      = make_uint4(base, count, depth, 0u);
+        uint64_t valid      = 0;
+        for (uint32_t k = 0; k < count; ++k) {
+            float r1, r2;
+            point(first + k, r1, r2);
+            Light_sample ls;
+            V3           c = v3(0.f, 0.f, 0.f);
+            float4       d = make_float4(0.f, 0.f, 1.f, 0.f);
+            if (sample_light<Media>(s, ps, n, total_sphere, pick_at(first + k), r1, r2, rng, ls)) {
+                V3 const e = eval(ls);
+                if (shading::max_component(e) > 0.f) {
+                    c = e;
+                    d = make_float4(ls.dir.x, ls.dir.y, ls.dir.z, ls.dist);
+                    valid |= 1ull << k;
+                }
+            }
+            p.pick_d[base + k] = d;
+            p.pick_c[base + k] = make_float4(c.x, c.y, c.z, __uint_as_float(rec));
+        }
+        if (valid != 0) {
+            uint32_t q = atomicAdd(out.count_shadow, uint32_t(__popcll(valid)));
+            for (uint32_t k = 0; k < count; ++k) {
+                if ((valid >> k) & 1u) {
+                    out.sq[q++] = Pick_shadow | (base + k);
+                }
             }
         }
-        return false;
-    };
-    uint32_t first = 0;
-    if (m > 1 && first0.light == Env_pick) {
-        shadow2 = slot(0, true);
-        first   = 1;
-    }
-    uint32_t const count = m - first;
-    if (count == 1) {
-        shadow = slot(first, false);
-    }
-    if (count < 2) {
         return;
     }
-    uint32_t const base = atomicAdd(out.count_picks, count);
-    uint32_t const rec  = atomicAdd(out.count_records, 1u);
-    p.split_o[rec]      = make_float4(ps.x, ps.y, ps.z, __uint_as_float(path));
-    p.split_m[rec]      = make_uint4(base, count, depth, 0u);
-    uint64_t valid      = 0;
-    for (uint32_t k = 0; k < count; ++k) {
+    uint32_t const first = m > 1 && first0.light == Env_pick ? 1u : 0u;  // lights of the second slot
+    uint32_t const count = m - first;
+    bool const     picks = count > 1;
+    uint32_t       base = 0, rec = 0;
+    if (picks) {
+        base           = atomicAdd(out.count_picks, count);
+        rec            = atomicAdd(out.count_records, 1u);
+        p.split_o[rec] = make_float4(ps.x, ps.y, ps.z, __uint_as_float(path));
+        p.split_m[rec] = make_uint4(base, count, depth, 0u);
+    }
+    // One body for every light, whatever becomes of its sample: copies of the light sampling and
+    // of eval would not fit the instruction cache.
+    uint64_t valid = 0;
+    for (uint32_t k = 0; k < m; ++k) {
         float r1, r2;
-        point(first + k, r1, r2);
-        Light_sample ls;
-        V3           c = v3(0.f, 0.f, 0.f);
-        float4       d = make_float4(0.f, 0.f, 1.f, 0.f);
-        if (sample_light(s, ps, n, total_sphere, pick_at(first + k), r1, r2, rng, ls)) {
+        point(k, r1, r2);
+        Light_pick const pk = k == 0 ? first0 : k == 1 ? first1 : light_at(s, ps, n, total_sphere, select, split, k);
+        Light_sample     ls;
+        V3               c  = v3(0.f, 0.f, 0.f);
+        bool             ok = false;
+        if (sample_light<Media>(s, ps, n, total_sphere, pk, r1, r2, rng, ls)) {
             V3 const e = eval(ls);
             if (shading::max_component(e) > 0.f) {
-                c = e;
-                d = make_float4(ls.dir.x, ls.dir.y, ls.dir.z, ls.dist);
-                valid |= 1ull << k;
+                c  = e;
+                ok = true;
             }
         }
-        p.pick_d[base + k] = d;
-        p.pick_c[base + k] = make_float4(c.x, c.y, c.z, __uint_as_float(rec));
+        if (k < first || !picks) {
+            if (ok) {
+                store_shadow(p, path, k < first, ps, ls, c, depth);
+                (k < first ? shadow2 : shadow) = true;
+            }
+        } else {
+            uint32_t const i = k - first;
+            p.pick_d[base + i] = ok ? make_float4(ls.dir.x, ls.dir.y, ls.dir.z, ls.dist) : make_float4(0.f, 0.f, 1.f, 0.f);
+            p.pick_c[base + i] = make_float4(c.x, c.y, c.z, __uint_as_float(rec));
+            valid |= uint64_t(ok) << i;
+        }
     }
     if (valid != 0) {
         uint32_t q = atomicAdd(out.count_shadow, uint32_t(__popcll(valid)));
@@ -2182,8 +2242,16 @@ __device__ float volume_light_pdf(Scene_gpu const& s, Paths const& p, uint32_t p
 }
 
 // ---- shade: one path vertex ----
+// Media: the scene has participating media.  Guided: path guiding.  Textured: some material has
+// maps.  A frame takes the variant without what it does not use (shade_kernel), and next_event has
+// one body for every light: the kernel waits on instruction fetch (4.0 of its 10 stalls an
+// instruction; 16.5 of 32 lanes, 2,700 instructions a warp, each fetched about once), so what
+// counts is the code a warp runs through.  512 x 512 x 64 Cornell frame 25.4 -> 23.3 ms, 960 x 540
+// x 32 instanced frame 85.5 -> 82.0 ms.  Blocks of 128 threads with registers for 5, 6 or 8 of them
+// on an SM (96, 80, 64) spill and are no faster.
+template <bool Media, bool Guided, bool Textured>
 __global__ void __launch_bounds__(Shade_block)
-    k_shade(Scene_gpu s, Launch const* __restrict__ launch, Paths p, uint32_t const* __restrict__ q_in,
+    k_shade(__grid_constant__ Scene_gpu const s, Launch const* __restrict__ launch, Paths p, uint32_t const* __restrict__ q_in,
             uint32_t const* __restrict__ count_in, Shade_out out) {
     Wave const&    wave = launch->wave;
     uint32_t const i   = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2200,7 +2268,7 @@ __global__ void __launch_bounds__(Shade_block)
         uint32_t vtx      = info & 0xFFu;
         uint32_t depth    = (info >> 8) & 0xFFu;
         bool     singular = (info >> 16) & 1u;
-        uint32_t medium   = info >> 17;  // material index + 1 of the medium the path is in
+        uint32_t medium   = Media ? info >> 17 : 0u;  // material index + 1 of the medium the path is in
         float4   T4       = p.T[path];
         V3       T        = f3v(T4);
         float    bsdf_pdf = T4.w;
@@ -2208,7 +2276,7 @@ __global__ void __launch_bounds__(Shade_block)
         V3       L        = f3v(L4);
         uint32_t const id = p.hit_id[path];
         bool     done     = false;
-        if (wave.record_depth) {
+        if (Guided && wave.record_depth) {
             // The training record of the previous vertex learns what its continuation found:
             // the radiance gathered so far (its own light samples included) marks the start.
             uint32_t const open = p.open_record[path];
@@ -2245,7 +2313,7 @@ __global__ void __launch_bounds__(Shade_block)
                 L = L + w * (T * v3(s.env.x, s.env.y, s.env.z));
             }
             done = true;
-        } else if (medium != 0) {
+        } else if (Media && medium != 0) {
             shading::Material const m = s.materials[medium - 1];
             V3 lw;
             bool const emissive = m.emission.x > 0.f || m.emission.y > 0.f || m.emission.z > 0.f;
@@ -2284,7 +2352,7 @@ __global__ void __launch_bounds__(Shade_block)
             }
         }
 
-        if (!done && scatter) {
+        if (Media && !done && scatter) {
             // Scattering vertex inside the medium (volumetric::Sample, HG phase function).
             if (depth >= wave.max_bounces) {
                 done = true;
@@ -2302,7 +2370,7 @@ __global__ void __launch_bounds__(Shade_block)
                 V3 const    pos = v3(ro.x + t_sc * rd.x, ro.y + t_sc * rd.y, ro.z + t_sc * rd.z);
                 V3 const    wo  = -dir_in;
                 float const select = rng.uniform();
-                next_event(s, p, wave, out, path, pos, v3(0.f, 0.f, 1.f), true, depth, select, rng, false, 0u,
+                next_event<Media, Guided>(s, p, wave, out, path, pos, v3(0.f, 0.f, 1.f), true, depth, select, rng, false, 0u,
                            0u, [&](Light_sample const& ls) {
                                float const f = shading::phase_hg(shading::dot(wo, ls.dir), g);
                                float const w = ls.pdf / (ls.pdf * ls.pdf + f * f);
@@ -2336,7 +2404,7 @@ __global__ void __launch_bounds__(Shade_block)
             V3 const     wo  = -dir_in;
             uint32_t const mat_id = wt.material;
             shading::Material mat = s.materials[mat_id];
-            if (mat.color_map | mat.surface_map) {
+            if (Textured && (mat.color_map | mat.surface_map)) {
                 float2 const t0  = s.uvs[wt.tri.x];
                 float2 const t1  = s.uvs[wt.tri.y];
                 float2 const t2  = s.uvs[wt.tri.z];
@@ -2389,7 +2457,7 @@ __global__ void __launch_bounds__(Shade_block)
                 done = true;
             }
 
-            if (!done && mat.type == shading::Type_volume) {
+            if (Media && !done && mat.type == shading::Type_volume) {
                 // Null boundary of a medium: the ray continues unchanged past the hit, the
                 // medium changes (interface_change), depth and MIS state are kept
                 // (pathtracer_mis.cpp:180-205, Straight_transmission).
@@ -2413,7 +2481,7 @@ __global__ void __launch_bounds__(Shade_block)
                 // The guide's mixture for this vertex (k_guide); continuation directions come
                 // from it with probability gf, else from the BSDF, and every pdf the MIS
                 // weights use is the combination of both.
-                bool const  guided = wave.guiding && depth < wave.guide_depth && p.guide_ok[i];
+                bool const  guided = Guided && wave.guiding && depth < wave.guide_depth && p.guide_ok[i];
                 float const gf     = !guided ? 0.f : (mat.metallic == 1.f ? wave.metal_fraction : wave.guide_fraction);
                 float4 const* const mix = reinterpret_cast<float4 const*>(p.guide_out + size_t(i) * Mixture_floats);
 
@@ -2429,9 +2497,9 @@ __global__ void __launch_bounds__(Shade_block)
                 V3 const    ps     = offset_ray(pos, geo_n);
                 float const select = golden ? golden_1d(wave, gpixel, gsample, golden_light_1d(depth, 0))
                                             : rng.uniform();
-                next_event(s, p, wave, out, path, ps, geo_n, false, depth, select, rng, golden, gpixel, gsample,
+                next_event<Media, Guided>(s, p, wave, out, path, ps, geo_n, false, depth, select, rng, golden, gpixel, gsample,
                            [&](Light_sample const& ls) {
-                               shading::Bxdf const f = shading::substitute_evaluate(mat, s.e_table, ctx, ls.dir);
+                               shading::Bxdf const f = shading::substitute_evaluate<!Guided>(mat, s.e_table, ctx, ls.dir);
                                float const pc = guided ? gf * mixture_pdf_at(mix, ls.dir) + (1.f - gf) * f.pdf
                                                        : f.pdf;
                                float const w  = ls.pdf / (ls.pdf * ls.pdf + pc * pc);
@@ -2524,6 +2592,18 @@ __global__ void __launch_bounds__(Shade_block)
     if (shadow2) {
         out.sq[sslot2] = path | Second_shadow;
     }
+}
+
+using Shade_kernel = void (*)(Scene_gpu const, Launch const*, Paths, uint32_t const*, uint32_t const*, Shade_out);
+
+Shade_kernel shade_kernel(bool media, bool guided, bool textured) {
+    if (media) {
+        return guided ? k_shade<true, true, true> : k_shade<true, false, true>;
+    }
+    if (guided) {
+        return textured ? k_shade<false, true, true> : k_shade<false, true, false>;
+    }
+    return textured ? k_shade<false, false, true> : k_shade<false, false, false>;
 }
 
 // ---- shadow rays through media: Worker::transmittance (rendering_worker.cpp:209-267) ----
@@ -4926,6 +5006,7 @@ int32_t Renderer::render(uint32_t first_sample, uint32_t num_samples) {
         return capture ? cudaEventRecordWithFlags(e, st, cudaEventRecordExternal) : cudaEventRecord(e, st);
     };
     bool const guide_at_all = settings_.guiding;
+    auto const shade        = shade_kernel(d_->has_media, guide_at_all, d_->textures != nullptr);
     auto const guided_at    = [&](uint32_t b) { return guide_at_all && (d_->has_media || b < settings_.guide_depth); };
 
     // Enqueues one wave's kernels (its launch block already copied to the device): generate,
@@ -4966,7 +5047,7 @@ int32_t Renderer::render(uint32_t first_sample, uint32_t num_samples) {
                     d_->paths, c, d_->net.weights(), d_->net.parameters(), ctr + Overflow_slot + 1);
                 SPB_RCUDA(record(guide_event(events++), capture));
             }
-            k_shade<<<(paths + Shade_block - 1) / Shade_block, Shade_block, 0, st>>>(
+            shade<<<(paths + Shade_block - 1) / Shade_block, Shade_block, 0, st>>>(
                 sg, d_->launch_dev, d_->paths, q_in, c,
                 Shade_out{q_out, c + Counter_stride, d_->shadow_queue, c + 1, c + 5, c + 6});
             if (d_->has_media) {
