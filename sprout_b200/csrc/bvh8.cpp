@@ -317,7 +317,7 @@ float hit_margin_for(double extent, double magnitude) {
 // fills the leaf record of primitive p.
 template <typename Emit>
 bool collapse_tree(std::vector<Box> const& boxes, std::vector<float> const& centroids,
-                   uint32_t num_threads, Wide_bvh& out, std::string& error, Emit&& emit) {
+                   uint32_t num_threads, Wide_bvh& out, std::string& error, float min_margin, Emit&& emit) {
     Binary_builder builder(boxes, centroids, num_threads);
     builder.build();
     auto&       bnodes = builder.nodes();
@@ -334,7 +334,7 @@ bool collapse_tree(std::vector<Box> const& boxes, std::vector<float> const& cent
     // A hit counts only if its point lies within the triangle's bounds widened by
     // hit_margin (2^-17 of the scene size); child boxes are widened by twice that, which
     // leaves hit_margin of room for the rounding of the traversal's slab arithmetic.
-    out.hit_margin   = hit_margin_for(extent, magnitude);
+    out.hit_margin   = std::max(hit_margin_for(extent, magnitude), min_margin);
     double const pad = 2.0 * double(out.hit_margin);
     double const scene_pad = scene_box_pad(extent, magnitude);
     for (int a = 0; a < 3; ++a) {
@@ -543,7 +543,7 @@ bool collapse_tree(std::vector<Box> const& boxes, std::vector<float> const& cent
 
 bool build_wide_bvh(uint32_t num_vertices, uint32_t num_triangles, float const* positions,
                     uint32_t const* indices, uint32_t num_threads, Wide_bvh& out,
-                    std::string& error, uint32_t const* tri_class) {
+                    std::string& error, uint32_t const* tri_class, float min_margin) {
     out = Wide_bvh();
 
     if (num_triangles == 0) {
@@ -581,7 +581,7 @@ bool build_wide_bvh(uint32_t num_vertices, uint32_t num_triangles, float const* 
         }
     }
 
-    return collapse_tree(boxes, centroids, num_threads, out, error,
+    return collapse_tree(boxes, centroids, num_threads, out, error, min_margin,
                          [&](uint32_t t, Wide_triangle& wt) {
                              float const* pa = positions + 3 * size_t(indices[3 * size_t(t) + 0]);
                              float const* pb = positions + 3 * size_t(indices[3 * size_t(t) + 1]);
@@ -616,7 +616,7 @@ bool build_wide_instances(uint32_t num_instances, float const* boxes_lo_hi, uint
             centroids[3 * size_t(i) + a] = 0.5f * (boxes[i].lo[a] + boxes[i].hi[a]);
         }
     }
-    return collapse_tree(boxes, centroids, num_threads, out, error,
+    return collapse_tree(boxes, centroids, num_threads, out, error, 0.f,
                          [&](uint32_t i, Wide_triangle& wt) {
                              wt.id        = i;
                              wt.tri_class = instance_class;

@@ -69,10 +69,13 @@ float hit_margin_for(double extent, double magnitude);
 constexpr uint32_t Max_wide_depth = 48;
 
 // Builds the 8-wide tree.  Returns false (with a message) if the input is unusable.
-// tri_class (optional, one word per triangle) is stored with each triangle.
+// tri_class (optional, one word per triangle) is stored with each triangle.  min_margin: the hit
+// margin is at least this (for a tree over some of a scene's triangles that is to answer as the
+// whole scene's tree does).
 bool build_wide_bvh(uint32_t num_vertices, uint32_t num_triangles, float const* positions,
                     uint32_t const* indices, uint32_t num_threads, Wide_bvh& out,
-                    std::string& error, uint32_t const* tri_class = nullptr);
+                    std::string& error, uint32_t const* tri_class = nullptr,
+                    float min_margin = 0.f);
 
 // Builds a top-level 8-wide tree over instance boxes (6 floats each: lo.xyz, hi.xyz).  Its leaf
 // records carry the instance index in Wide_triangle::id and instance_class in tri_class; their
