@@ -31,11 +31,20 @@ namespace spb {
 
 namespace {
 
+struct Uninitialised {};
+
 struct Box {
-    float lo[3] = {std::numeric_limits<float>::max(), std::numeric_limits<float>::max(),
-                   std::numeric_limits<float>::max()};
-    float hi[3] = {-std::numeric_limits<float>::max(), -std::numeric_limits<float>::max(),
-                   -std::numeric_limits<float>::max()};
+    float lo[3];
+    float hi[3];
+
+    Box() {
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = std::numeric_limits<float>::max();
+            hi[a] = -std::numeric_limits<float>::max();
+        }
+    }
+
+    explicit Box(Uninitialised) {}
 
     void grow(Box const& b) {
         for (int a = 0; a < 3; ++a) {
@@ -74,7 +83,9 @@ struct Binary_node {
 };
 
 constexpr uint32_t Num_bins             = 32;
-constexpr uint32_t Parallel_threshold   = 1u << 15;
+// Subtrees from this size on may be built by a thread of their own: one of 4,096 triangles takes
+// about a millisecond, starting a thread a few hundredths.
+constexpr uint32_t Parallel_threshold   = 1u << 12;
 constexpr uint32_t Max_leaf_triangles   = 3;
 // The collapse does not open a child holding at most Keep_leaf triangles: it stays one leaf
 // slot of up to Keep_leaf triangles (0: every binary child with more than one triangle can be
@@ -123,8 +134,8 @@ class Binary_builder {
   private:
     struct Bin {
         Box      box;
-        Box      cbox;
-        uint32_t count = 0;
+        uint32_t count;
+        Bin() : box(Uninitialised()) {}
     };
 
     void build(uint32_t node_id, uint32_t begin, uint32_t end, Box const& box, Box const& cbox,
@@ -186,7 +197,11 @@ class Binary_builder {
         int   best_axis = -1;
         int   best_bin  = 0;
 
-        Bin bins[3][Num_bins];
+        // Only the bins that a primitive falls into are set up and looked at (used: their bits).
+        // Most nodes hold a few primitives, and going through all 96 bins for each was two thirds
+        // of the build.  Bins without a primitive would change no box, count or cost.
+        Bin      bins[3][Num_bins];
+        uint32_t used[3] = {0, 0, 0};
 
         float scale[3];
         for (int a = 0; a < 3; ++a) {
@@ -202,9 +217,13 @@ class Binary_builder {
                     continue;
                 }
                 uint32_t const b = bin_of(c[a], cbox.lo[a], scale[a]);
+                if (!(used[a] >> b & 1u)) {
+                    used[a] |= 1u << b;
+                    bins[a][b].box   = Box();
+                    bins[a][b].count = 0;
+                }
                 bins[a][b].count++;
                 bins[a][b].box.grow(boxes_[p]);
-                bins[a][b].cbox.grow(c);
             }
         }
 
@@ -216,7 +235,10 @@ class Binary_builder {
             uint32_t right_count[Num_bins];
             Box      acc;
             uint32_t cnt = 0;
-            for (int b = int(Num_bins) - 1; b > 0; --b) {
+            // right_*[b]: the used bins from b on
+            for (uint32_t rest = used[a]; rest != 0;) {
+                uint32_t const b = 31u - uint32_t(__builtin_clz(rest));
+                rest &= ~(1u << b);
                 acc.grow(bins[a][b].box);
                 cnt += bins[a][b].count;
                 right_area[b]  = acc.area();
@@ -224,17 +246,18 @@ class Binary_builder {
             }
             acc = Box();
             cnt = 0;
-            for (uint32_t b = 1; b < Num_bins; ++b) {
-                acc.grow(bins[a][b - 1].box);
-                cnt += bins[a][b - 1].count;
-                if (cnt == 0 || right_count[b] == 0) {
-                    continue;
-                }
-                float const cost = acc.area() * float(cnt) + right_area[b] * float(right_count[b]);
+            // Splits after each used bin but the last; the split lies directly behind the bin.
+            for (uint32_t rest = used[a]; (rest & (rest - 1)) != 0;) {
+                uint32_t const l = uint32_t(__builtin_ctz(rest));
+                rest &= rest - 1;
+                uint32_t const r = uint32_t(__builtin_ctz(rest));
+                acc.grow(bins[a][l].box);
+                cnt += bins[a][l].count;
+                float const cost = acc.area() * float(cnt) + right_area[r] * float(right_count[r]);
                 if (cost < best_cost) {
                     best_cost = cost;
                     best_axis = a;
-                    best_bin  = int(b);
+                    best_bin  = int(l) + 1;
                 }
             }
         }
@@ -252,13 +275,12 @@ class Binary_builder {
                                                               sc)) < best_bin;
                                         });
         mid = uint32_t(it - prims_.data());
-        for (int b = 0; b < best_bin; ++b) {
-            lbox.grow(bins[a][b].box);
-            lcbox.grow(bins[a][b].cbox);
+        for (uint32_t rest = used[a]; rest != 0; rest &= rest - 1) {
+            int const b = __builtin_ctz(rest);
+            (b < best_bin ? lbox : rbox).grow(bins[a][b].box);
         }
-        for (int b = best_bin; b < int(Num_bins); ++b) {
-            rbox.grow(bins[a][b].box);
-            rcbox.grow(bins[a][b].cbox);
+        for (uint32_t i = begin; i < end; ++i) {
+            (i < mid ? lcbox : rcbox).grow(&centroids_[3 * size_t(prims_[i])]);
         }
         return mid > begin && mid < end;
     }
