@@ -422,7 +422,7 @@ def main():
         e_el = max_over_ranks(time.perf_counter() - t0, dist, "cuda")
         e2e = {"value": round(world * args.rays * e_steps / e_el / 1e6, 3), "unit": "Mrays/s",
                "h2d_bytes_per_step": 32 * args.rays, "d2h_bytes_per_step": 8 * args.rays,
-               "steps": e_steps, "path": "spb_intersect_host (pinned host buffers, 2-stream chunked copies)"}
+               "steps": e_steps, "path": "spb_intersect_host (pinned host buffers, 3-stream chunked copies)"}
 
     value = world * args.rays * args.steps / elapsed / 1e6
     mean_kernel_s = statistics.mean(kernel_ms) / 1e3

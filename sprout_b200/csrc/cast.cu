@@ -63,8 +63,8 @@ constexpr uint32_t Full_mask        = 0xFFFFFFFFu;
 constexpr uint32_t Waiting          = 64;  // rays a warp of the sparse form fetches together
 
 // Counter slots (2 words each: work counter, overflow count).  Slot 0 serves the device
-// entry points, slots 1 and 2 the two streams of the host pipeline.
-constexpr uint32_t Num_counter_slots = 3;
+// entry points, slots 1 to 3 the three streams of the host pipeline.
+constexpr uint32_t Num_counter_slots = 4;
 // After them, one word a slot: the form of kernel its cast takes (choose_kernel).
 constexpr uint32_t Num_counter_words = 3 * Num_counter_slots;
 
@@ -265,14 +265,15 @@ __global__ void SPB_CAST_BOUNDS
 }
 
 struct Pipeline {
-    static constexpr uint64_t Chunk = 1ull << 21;  // rays per chunk
+    static constexpr uint64_t Chunk   = 1ull << 20;  // most rays per chunk
+    static constexpr int      Streams = 3;
 
-    cudaStream_t streams[2] = {nullptr, nullptr};
-    float4*      rays[2]    = {nullptr, nullptr};
-    uint32_t*    ids[2]     = {nullptr, nullptr};
-    float*       ts[2]      = {nullptr, nullptr};
-    float2*      uvs[2]     = {nullptr, nullptr};
-    uint8_t*     occ[2]     = {nullptr, nullptr};
+    cudaStream_t streams[Streams] = {};
+    float4*      rays[Streams]    = {};
+    uint32_t*    ids[Streams]     = {};
+    float*       ts[Streams]      = {};
+    float2*      uvs[Streams]     = {};
+    uint8_t*     occ[Streams]     = {};
     bool         ready      = false;
 };
 
@@ -331,7 +332,7 @@ class Device_scope {
 };
 
 void free_pipeline(Pipeline& p) {
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < Pipeline::Streams; ++s) {
         cudaFree(p.rays[s]);
         cudaFree(p.ids[s]);
         cudaFree(p.ts[s]);
@@ -349,7 +350,7 @@ int32_t ensure_pipeline(spb_tree* tree) {
     if (p.ready) {
         return SPB_OK;
     }
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < Pipeline::Streams; ++s) {
         SPB_CUDA(cudaStreamCreateWithFlags(&p.streams[s], cudaStreamNonBlocking));
         SPB_CUDA(cudaMalloc(&p.rays[s], Pipeline::Chunk * 32));
         SPB_CUDA(cudaMalloc(&p.ids[s], Pipeline::Chunk * 4));
@@ -620,11 +621,18 @@ int32_t cast_host(spb_tree* tree, bool any_hit, float const* rays, uint64_t n, u
         return s;
     }
     Pipeline& p = tree->pipe;
-    uint64_t const chunks = (n + Pipeline::Chunk - 1) / Pipeline::Chunk;
+    // An eighth of the batch at a time, so that the copies in, the casts and the copies out
+    // overlap: the call then takes little more than its copies in.  Chunks below 65,536 rays would
+    // not fill the GPU.  Three streams: with two, a chunk's copy in waits for the copy out before last.
+    // (1,000,003 rays from pinned memory, 262,144 triangles: 910 us in one
+    // chunk, 887 in eight with two streams, 760 with three.)
+    uint64_t const eighth = (n / 8 + 32767) / 32768 * 32768;
+    uint64_t const chunk  = std::clamp<uint64_t>(eighth, 65536, Pipeline::Chunk);
+    uint64_t const chunks = (n + chunk - 1) / chunk;
     for (uint64_t c = 0; c < chunks; ++c) {
-        int const          s     = int(c & 1);
-        uint64_t const     first = c * Pipeline::Chunk;
-        uint64_t const     count = std::min<uint64_t>(Pipeline::Chunk, n - first);
+        int const          s     = int(c % Pipeline::Streams);
+        uint64_t const     first = c * chunk;
+        uint64_t const     count = std::min<uint64_t>(chunk, n - first);
         cudaStream_t const st    = p.streams[s];
         SPB_CUDA(cudaMemcpyAsync(p.rays[s], rays + 8 * first, count * 32, cudaMemcpyHostToDevice,
                                  st));
@@ -644,9 +652,10 @@ int32_t cast_host(spb_tree* tree, bool any_hit, float const* rays, uint64_t n, u
             }
         }
     }
-    SPB_CUDA(cudaStreamSynchronize(p.streams[0]));
-    SPB_CUDA(cudaStreamSynchronize(p.streams[1]));
-    tree->last_stream = p.streams[1];
+    for (cudaStream_t const st : p.streams) {
+        SPB_CUDA(cudaStreamSynchronize(st));
+    }
+    tree->last_stream = p.streams[Pipeline::Streams - 1];
     return SPB_OK;
 }
 
@@ -687,7 +696,10 @@ extern "C" SPB_API int32_t spb_tree_status(spb_tree* tree, uint32_t* overflowed_
     SPB_CUDA(cudaDeviceSynchronize());
     uint32_t host[2 * Num_counter_slots];
     SPB_CUDA(cudaMemcpy(host, tree->d_counters, sizeof(host), cudaMemcpyDeviceToHost));
-    *overflowed_rays = host[1] + host[3] + host[5];
+    *overflowed_rays = 0;
+    for (uint32_t slot = 0; slot < Num_counter_slots; ++slot) {
+        *overflowed_rays += host[2 * slot + 1];
+    }
     return SPB_OK;
 }
 
