@@ -526,34 +526,6 @@ __device__ __forceinline__ bool spent(Traversal const& tv, Instance_state const*
     return s;
 }
 
-// One traversal step of a lane by itself: a triangle if the current triangle group has one
-// pending, else the next node.  Returns true when the ray is finished (any hit found, or nothing
-// left to visit).  For callers whose lanes are not together (see warp_step).
-template <bool Any_hit, bool Filter = false, bool Instances = false>
-__device__ __forceinline__ bool traversal_step(Ray_state& r, Traversal& tv, uint2* stack,
-                                               Wide_node const* __restrict__ nodes,
-                                               float4 const* __restrict__ triangles,
-                                               float hit_margin, uint32_t* overflow,
-                                               uint32_t skip_class = 0,
-                                               Instance_state* is = nullptr,
-                                               Instance_trace const* __restrict__ instances = nullptr) {
-    // Single exit (no early return): the place where the two branches rejoin decides where a
-    // diverged warp reconverges, and keeping it at the end measured fastest.
-    bool done = false;
-    if (tv.tri_group.y != 0) {
-        done = triangle_step<Any_hit, Filter, Instances>(r, tv, stack, triangles, hit_margin, overflow, skip_class,
-                                                         is, instances);
-    } else {
-        next_group<Instances>(r, tv, stack, is);
-        if (tv.group.y & 0xFF000000u) {
-            done = node_step(r, tv, stack, nodes, overflow);
-        } else if (!Instances || tv.tri_group.y == 0) {
-            done = true;
-        }
-    }
-    return done;
-}
-
 // One traversal step of a whole warp (all 32 lanes call it; inactive ones pass active = false and
 // only take part in the convergence barriers): every lane tests a pending triangle, if it has
 // one, then, if it has none left, visits its next node.  The barriers hold the lanes together at
