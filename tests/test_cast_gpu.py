@@ -247,3 +247,46 @@ def test_every_launch_rule_bit_exact(torch_cuda, count, extent):
     hit = want["ids"] != MISS
     assert np.array_equal(_bits(uv.cpu().numpy()[hit]), _bits(want["uv"][hit]))
     assert np.array_equal(occ.cpu().numpy(), want["occluded"])
+
+
+def _pinned(torch, a):
+    t = torch.empty(a.shape, dtype=torch.uint8 if a.dtype == np.uint8 else torch.float32, pin_memory=True)
+    out = t.numpy().view(a.dtype)
+    out[...] = a
+    return out
+
+
+# Batches about the host pipeline's rules: one chunk, a stream's buffers used again (the fourth
+# chunk on), short last chunks, the smallest chunks of page-locked (65,536) and pageable rays
+# (131,072), and chunks so large that each chooses its form of the kernel (2^20).
+HOST_SIZES = [65536, 65537, 3 * 65536, 3 * 65536 + 1, 131072 + 1, 4 * 65536 + 33, 1000003, (8 << 20) + 33]
+
+
+@pytest.mark.parametrize("rays_at,results_at", [("pageable", "pageable"), ("pinned", "pinned"),
+                                                ("pinned", "pageable"), ("pageable", "pinned")])
+@pytest.mark.parametrize("count", HOST_SIZES)
+def test_host_pipeline_answers_as_the_device_entry_points(torch_cuda, count, rays_at, results_at):
+    """Closest hits with and without barycentrics and any hits of two batches through one tree,
+    against the device entry points (which the tests above hold to the restatement)."""
+    torch = torch_cuda
+    place = {"pageable": lambda a: a, "pinned": lambda a: _pinned(torch, a)}
+    pos, idx = oracle.synth_sphere_mesh(8, 0.1, 1)
+    with sb.Tree() as tree:
+        tree.build(pos, idx)
+        for seed, extent in ((5, 0.5), (6, 6.0)):
+            rays = place[rays_at](sb.random_rays(count, seed=seed, extent=extent))
+            at = torch.from_numpy(rays).cuda()
+            want = [x.cpu().numpy() for x in tree.intersect(at, want_uv=True)] + [tree.intersect_p(at).cpu().numpy()]
+            new = place[results_at]
+            ids, t = new(np.full(count, 7, np.uint32)), new(np.full(count, -1.0, np.float32))
+            uv, occ = new(np.full((count, 2), -1.0, np.float32)), new(np.full(count, 9, np.uint8))
+            tree.intersect(rays, out=(ids, t, uv), want_uv=True)
+            assert np.array_equal(ids, want[0].view(np.uint32))
+            assert np.array_equal(_bits(t), _bits(want[1]))
+            assert np.array_equal(_bits(uv), _bits(want[2]))
+            ids[:], t[:] = 7, -1.0
+            tree.intersect(rays, out=(ids, t, None))
+            assert np.array_equal(ids, want[0].view(np.uint32)) and np.array_equal(_bits(t), _bits(want[1]))
+            tree.intersect_p(rays, out=occ)
+            assert np.array_equal(occ, want[3])
+        assert tree.status() == 0
