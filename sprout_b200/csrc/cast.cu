@@ -385,7 +385,8 @@ int32_t launch(spb_tree* tree, bool any_hit, uint32_t slot, float4 const* rays, 
             tree->scene_lo, tree->scene_hi, nullptr);
     };
     uint32_t const* form = nullptr;
-    if (n >= Choose_rays) {
+    // (The sparse form takes more rays at a time than a fixed share holds: it needs the counter.)
+    if (work && n >= Choose_rays) {
         uint32_t* const chosen = tree->d_counters + 2 * Num_counter_slots + slot;
         choose_kernel<<<1, Probes, 0, stream>>>(rays, n, tree->scene_lo, tree->scene_hi, chosen);
         form = chosen;
