@@ -67,7 +67,8 @@ constexpr uint32_t Class_instance   = 4;  // ... of top-level leaves (instances)
 // Counter block (uint32): per bounce b, at Counter_stride * b + k: k = 0 extension count,
 // 1 shadow count, 2 extend fetch, 3 shadow fetch, 4 shadow slots through media (rays to
 // emitters), 5 picks of split light selections, 6 split records, 7 picks through media,
-// 8 shadow slots through media (rays to the environment); then the overflow counter.
+// 8 shadow slots through media (rays to the environment), 9 and 10 k_transmit's fetch of shadow
+// slots and of picks, 11 k_track's fetch; then the overflow counter.
 constexpr uint32_t Counter_stride = 16;
 constexpr uint32_t Graph_max_paths = 1u << 25;  // largest wave replayed from a CUDA graph
 constexpr uint64_t Pick_budget     = 24ull << 30;  // bytes of picks a wave may hold
@@ -275,7 +276,7 @@ struct Paths {
     uint8_t*  guide_ok;
     float4*   rec;
     uint32_t* open_record;
-    // Scenes with media: what k_track found for a path inside a grid (path weight, distance).
+    // Scenes with grids that k_track takes: what it found for a path inside one (path weight, distance).
     float4*   track;
 };
 
@@ -2203,10 +2204,10 @@ __device__ float volume_light_pdf(Scene_gpu const& s, Paths const& p, uint32_t p
 
 // Whether k_track takes the paths inside a material's medium: density and colour grids that do not
 // emit.
-__device__ __forceinline__ bool emits(shading::Material const& m) {
+SPB_HD bool emits(shading::Material const& m) {
     return m.emission.x > 0.f || m.emission.y > 0.f || m.emission.z > 0.f;
 }
-__device__ __forceinline__ bool grid_tracked(shading::Material const& m) { return m.medium != 0 && !emits(m); }
+SPB_HD bool grid_tracked(shading::Material const& m) { return m.medium != 0 && !emits(m); }
 
 // ---- track: paths inside density grids, to their next event ----
 // Delta tracking with spectral MIS from a path's vertex to its next surface
@@ -3921,6 +3922,7 @@ struct Renderer::Device {
     uint32_t* counters       = nullptr;
     uint32_t* pinned_count   = nullptr;  // host-pinned word for the queue-length check
     bool      has_media      = false;
+    bool      tracks_media   = false;  // ... some of them grids that k_track takes
     // split light selection: the most lights one selection returns in this scene, the depth
     // the split walk starts at, and the picks the buffers hold
     uint32_t  max_picks        = 1;
@@ -4325,6 +4327,7 @@ int32_t Renderer::set_scene(Scene_desc const& scene, uint32_t num_threads) {
     // A new scene is tuned anew, at the occupancy of the traversal it uses.
     d_->tuner.reset(two_level ? d_->per_sm_inst : d_->per_sm_flat);
     d_->has_media      = false;
+    d_->tracks_media   = false;
     d_->spectral_scene = !two_level;
 
     std::vector<Wide_node>           nodes;
@@ -4670,6 +4673,9 @@ int32_t Renderer::set_scene(Scene_desc const& scene, uint32_t num_threads) {
     cudaDeviceSynchronize();
     SPB_RCUDA(upload(d_->nodes, nodes.data(), nodes.size() * sizeof(Wide_node)));
     d_->boundary_root = boundary_root;
+    for (shading::Material const& m : scene.materials) {
+        d_->tracks_media |= d_->has_media && m.type == shading::Type_volume && grid_tracked(m);
+    }
     SPB_RCUDA(upload(d_->tris, tris.data(), tris.size() * sizeof(Wide_triangle)));
     SPB_RCUDA(upload(d_->inst_shade, shade.data(), shade.size() * sizeof(Instance_shade)));
     SPB_RCUDA(upload(d_->inst_materials, inst_materials.data(), inst_materials.size() * sizeof(uint32_t)));
@@ -5059,7 +5065,7 @@ int32_t Renderer::start_frame() {
 
 int32_t Renderer::ensure_buffers(uint32_t paths, uint32_t picks_per_path) {
     uint64_t const picks = uint64_t(paths) * picks_per_path;
-    if (paths <= d_->capacity && picks <= d_->pick_capacity && (d_->paths.track || !d_->has_media)) {
+    if (paths <= d_->capacity && picks <= d_->pick_capacity && (d_->paths.track || !d_->tracks_media)) {
         return SPB_OK;
     }
     clear_graphs();
@@ -5119,7 +5125,7 @@ int32_t Renderer::ensure_buffers(uint32_t paths, uint32_t picks_per_path) {
     SPB_RCUDA(dev_malloc(&p.sh2_L, n * sizeof(float4)));
     SPB_RCUDA(dev_malloc(&p.prev_n, n * sizeof(float4)));
     SPB_RCUDA(dev_malloc(&p.L2, n * sizeof(float4)));
-    if (d_->has_media) {
+    if (d_->tracks_media) {
         SPB_RCUDA(dev_malloc(&p.track, n * sizeof(float4)));
     }
     SPB_RCUDA(dev_malloc(&d_->queue[0], n * sizeof(uint32_t)));
@@ -5514,7 +5520,7 @@ int32_t Renderer::render(uint32_t first_sample, uint32_t num_samples) {
                     d_->paths, c, d_->net.weights(), d_->net.parameters(), ctr + Overflow_slot + 1);
                 SPB_RCUDA(record(guide_event(events++), capture));
             }
-            if (d_->has_media) {
+            if (d_->tracks_media) {
                 k_track<<<std::min((paths + Trace_block - 1) / Trace_block, d_->track_grid), Trace_block, 0, st>>>(
                     sg, d_->paths, q_in, c, c + 11);
             }
