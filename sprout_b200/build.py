@@ -26,7 +26,7 @@ SOURCES = ["common.cpp", "synth.cpp", "bvh8.cpp", "ggx_table.cpp", "light_tree.c
            "cast.cu",
            "guide.cu", "render.cu", "capi.cpp"]
 HEADERS = ["common.hpp", "bvh8.hpp", "traverse.cuh", "material.cuh", "render.hpp", "json.hpp", "ggx_table.hpp",
-           "light_tree.hpp", "guide.cuh", "guide_mlp.cuh", "guide.hpp", "tuner.hpp", "postprocess.hpp", "image_io.hpp",
+           "light_tree.hpp", "guide.cuh", "guide_mlp.cuh", "guide.hpp", "tuner.hpp", "buffers.hpp", "postprocess.hpp", "image_io.hpp",
            "spectral.cuh"]
 
 NVCC_FLAGS = [

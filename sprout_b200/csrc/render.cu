@@ -30,6 +30,7 @@
 #include <cstring>
 #include <map>
 
+#include "buffers.hpp"
 #include "bvh8.hpp"
 #include "common.hpp"
 #include "ggx_table.hpp"
@@ -3989,6 +3990,12 @@ void free_ptr(T*& p) {
     }
 }
 
+// All buffers of the set released, then allocated anew (replace_buffers).
+cudaError_t replace(std::vector<Buffer> const& set) {
+    return cudaError_t(replace_buffers(
+        set, [](void** p, size_t bytes) { return pool_malloc(p, bytes); }, [](void* p) { free_ptr(p); }));
+}
+
 template <typename T>
 cudaError_t upload(T*& dst, void const* src, size_t bytes) {
     free_ptr(dst);
@@ -5041,12 +5048,10 @@ int32_t Renderer::set_views(std::vector<Camera_desc> const& views) {
     d_->traced_pixels = traced.back();
     uint32_t const pixels = film.back();
     if (pixels != d_->film_pixels) {
-        free_ptr(d_->film);
-        free_ptr(d_->comp);
-        free_ptr(d_->out);
-        SPB_RCUDA(dev_malloc(&d_->film, pixels * sizeof(float4)));
-        SPB_RCUDA(dev_malloc(&d_->comp, pixels * sizeof(float4)));
-        SPB_RCUDA(dev_malloc(&d_->out, pixels * sizeof(float4)));
+        size_t const bytes = pixels * sizeof(float4);
+        d_->film_pixels = 0;
+        camera_ready_   = false;
+        SPB_RCUDA(replace({buffer(d_->film, bytes), buffer(d_->comp, bytes), buffer(d_->out, bytes)}));
         d_->film_pixels = pixels;
     }
     camera_ready_ = true;
@@ -5069,82 +5074,55 @@ int32_t Renderer::ensure_buffers(uint32_t paths, uint32_t picks_per_path) {
         return SPB_OK;
     }
     clear_graphs();
-    Paths& p = d_->paths;
-    free_ptr(p.ray_o);
-    free_ptr(p.ray_d);
-    free_ptr(p.hit_id);
-    free_ptr(p.hit_inst);
-    free_ptr(p.hit_t);
-    free_ptr(p.hit_uv);
-    free_ptr(p.T);
-    free_ptr(p.L);
-    free_ptr(p.puv);
-    free_ptr(p.rng);
-    free_ptr(p.info);
-    free_ptr(p.sh_o);
-    free_ptr(p.sh_d);
-    free_ptr(p.sh_L);
-    free_ptr(p.prev_n);
-    free_ptr(p.split_o);
-    free_ptr(p.sh2_o);
-    free_ptr(p.sh2_d);
-    free_ptr(p.sh2_L);
-    free_ptr(p.split_m);
-    free_ptr(p.pick_d);
-    free_ptr(p.pick_c);
-    free_ptr(p.L2);
-    free_ptr(p.track);
-    free_ptr(p.guide_in);
-    free_ptr(p.guide_out);
-    free_ptr(p.guide_ok);
-    free_ptr(p.rec);
-    free_ptr(p.open_record);
-    d_->guide_paths = 0;
-    free_ptr(d_->queue[0]);
-    free_ptr(d_->queue[1]);
-    free_ptr(d_->shadow_queue);
-    free_ptr(d_->transmit_queue);
-    free_ptr(d_->transmit_pick_queue);
+    Paths&       p = d_->paths;
     size_t const n = paths;
-    SPB_RCUDA(dev_malloc(&p.ray_o, n * sizeof(float4)));
-    SPB_RCUDA(dev_malloc(&p.ray_d, n * sizeof(float4)));
-    SPB_RCUDA(dev_malloc(&p.hit_id, n * sizeof(uint32_t)));
-    SPB_RCUDA(dev_malloc(&p.hit_inst, n * sizeof(uint32_t)));
-    SPB_RCUDA(dev_malloc(&p.hit_t, n * sizeof(float)));
-    SPB_RCUDA(dev_malloc(&p.hit_uv, n * sizeof(float2)));
-    SPB_RCUDA(dev_malloc(&p.T, n * sizeof(float4)));
-    SPB_RCUDA(dev_malloc(&p.L, n * sizeof(float4)));
-    SPB_RCUDA(dev_malloc(&p.puv, n * sizeof(float2)));
-    SPB_RCUDA(dev_malloc(&p.rng, n * sizeof(uint4)));
-    SPB_RCUDA(dev_malloc(&p.info, n * sizeof(uint32_t)));
-    SPB_RCUDA(dev_malloc(&p.sh_o, n * sizeof(float4)));
-    SPB_RCUDA(dev_malloc(&p.sh_d, n * sizeof(float4)));
-    SPB_RCUDA(dev_malloc(&p.sh_L, n * sizeof(float4)));
-    SPB_RCUDA(dev_malloc(&p.sh2_o, n * sizeof(float4)));
-    SPB_RCUDA(dev_malloc(&p.sh2_d, n * sizeof(float4)));
-    SPB_RCUDA(dev_malloc(&p.sh2_L, n * sizeof(float4)));
-    SPB_RCUDA(dev_malloc(&p.prev_n, n * sizeof(float4)));
-    SPB_RCUDA(dev_malloc(&p.L2, n * sizeof(float4)));
-    if (d_->tracks_media) {
-        SPB_RCUDA(dev_malloc(&p.track, n * sizeof(float4)));
-    }
-    SPB_RCUDA(dev_malloc(&d_->queue[0], n * sizeof(uint32_t)));
-    SPB_RCUDA(dev_malloc(&d_->queue[1], n * sizeof(uint32_t)));
     // Split selections: a record per path and every light its selection can return.  Shadow
     // rays: a path's two slots and every pick.
     size_t const np = std::max<size_t>(size_t(n) * picks_per_path, 1);
-    SPB_RCUDA(dev_malloc(&p.split_o, n * sizeof(float4)));
-    SPB_RCUDA(dev_malloc(&p.split_m, n * sizeof(uint4)));
-    SPB_RCUDA(dev_malloc(&p.pick_d, np * sizeof(float4)));
-    SPB_RCUDA(dev_malloc(&p.pick_c, np * sizeof(float4)));
-    SPB_RCUDA(dev_malloc(&d_->shadow_queue, (2 * n + np) * sizeof(uint32_t)));
-    SPB_RCUDA(dev_malloc(&d_->transmit_queue, 2 * n * sizeof(uint32_t)));
-    SPB_RCUDA(dev_malloc(&d_->transmit_pick_queue, np * sizeof(uint32_t)));
-    d_->pick_capacity = uint64_t(n) * picks_per_path;
+    d_->capacity      = 0;
+    d_->pick_capacity = 0;
+    d_->guide_paths   = 0;
+    SPB_RCUDA(replace({
+        buffer(p.ray_o, n * sizeof(float4)),
+        buffer(p.ray_d, n * sizeof(float4)),
+        buffer(p.hit_id, n * sizeof(uint32_t)),
+        buffer(p.hit_inst, n * sizeof(uint32_t)),
+        buffer(p.hit_t, n * sizeof(float)),
+        buffer(p.hit_uv, n * sizeof(float2)),
+        buffer(p.T, n * sizeof(float4)),
+        buffer(p.L, n * sizeof(float4)),
+        buffer(p.puv, n * sizeof(float2)),
+        buffer(p.rng, n * sizeof(uint4)),
+        buffer(p.info, n * sizeof(uint32_t)),
+        buffer(p.sh_o, n * sizeof(float4)),
+        buffer(p.sh_d, n * sizeof(float4)),
+        buffer(p.sh_L, n * sizeof(float4)),
+        buffer(p.sh2_o, n * sizeof(float4)),
+        buffer(p.sh2_d, n * sizeof(float4)),
+        buffer(p.sh2_L, n * sizeof(float4)),
+        buffer(p.prev_n, n * sizeof(float4)),
+        buffer(p.L2, n * sizeof(float4)),
+        buffer(p.track, d_->tracks_media ? n * sizeof(float4) : 0),
+        buffer(p.guide_in, 0),  // (ensure_guide)
+        buffer(p.guide_out, 0),
+        buffer(p.guide_ok, 0),
+        buffer(p.rec, 0),
+        buffer(p.open_record, 0),
+        buffer(d_->queue[0], n * sizeof(uint32_t)),
+        buffer(d_->queue[1], n * sizeof(uint32_t)),
+        buffer(p.split_o, n * sizeof(float4)),
+        buffer(p.split_m, n * sizeof(uint4)),
+        buffer(p.pick_d, np * sizeof(float4)),
+        buffer(p.pick_c, np * sizeof(float4)),
+        buffer(d_->shadow_queue, (2 * n + np) * sizeof(uint32_t)),
+        buffer(d_->transmit_queue, 2 * n * sizeof(uint32_t)),
+        buffer(d_->transmit_pick_queue, np * sizeof(uint32_t)),
+    }));
     if (!d_->counters) {
         SPB_RCUDA(dev_malloc(&d_->counters, Counter_words * sizeof(uint32_t)));
     }
-    d_->capacity = paths;
+    d_->pick_capacity = uint64_t(n) * picks_per_path;
+    d_->capacity      = paths;
     return SPB_OK;
 }
 
@@ -5155,35 +5133,32 @@ int32_t Renderer::ensure_guide(uint32_t paths) {
     uint32_t const rd = settings_.record_depth;
     if (d_->guide_paths < paths || d_->guide_records != rd) {
         clear_graphs();
-        free_ptr(p.guide_in);
-        free_ptr(p.guide_out);
-        free_ptr(p.guide_ok);
-        free_ptr(p.rec);
-        free_ptr(p.open_record);
         size_t const n = d_->capacity;
         size_t const tiled_entries = (n + guide::Tile - 1) / guide::Tile * guide::Tile;
-        SPB_RCUDA(dev_malloc(&p.guide_in, tiled_entries * guide::Inputs * sizeof(__nv_bfloat16)));
-        SPB_RCUDA(dev_malloc(&p.guide_out, n * Mixture_floats * sizeof(float)));
-        SPB_RCUDA(dev_malloc(&p.guide_ok, n));
-        SPB_RCUDA(dev_malloc(&p.rec, n * rd * Record_float4 * sizeof(float4)));
-        SPB_RCUDA(dev_malloc(&p.open_record, n * sizeof(uint32_t)));
+        d_->guide_paths = 0;
+        SPB_RCUDA(replace({
+            buffer(p.guide_in, tiled_entries * guide::Inputs * sizeof(__nv_bfloat16)),
+            buffer(p.guide_out, n * Mixture_floats * sizeof(float)),
+            buffer(p.guide_ok, n),
+            buffer(p.rec, n * rd * Record_float4 * sizeof(float4)),
+            buffer(p.open_record, n * sizeof(uint32_t)),
+        }));
         d_->guide_paths   = uint32_t(n);
         d_->guide_records = rd;
     }
     uint32_t const batch = settings_.guide_batch;
     if (d_->train_capacity < batch) {
-        free_ptr(d_->train_in);
-        free_ptr(d_->train_dir);
-        free_ptr(d_->train_w);
-        free_ptr(d_->train_parts);
         size_t const rows = (size_t(batch) + guide::Tile - 1) / guide::Tile * guide::Tile;
-        SPB_RCUDA(dev_malloc(&d_->train_in, rows * guide::Inputs * sizeof(__nv_bfloat16)));
-        SPB_RCUDA(dev_malloc(&d_->train_dir, size_t(batch) * 3 * sizeof(float)));
-        SPB_RCUDA(dev_malloc(&d_->train_w, size_t(batch) * sizeof(float)));
-        SPB_RCUDA(dev_malloc(&d_->train_parts, (rows + 255) / 256 * sizeof(float)));
-        d_->train_capacity = batch;
+        d_->train_capacity = 0;
+        SPB_RCUDA(replace({
+            buffer(d_->train_in, rows * guide::Inputs * sizeof(__nv_bfloat16)),
+            buffer(d_->train_dir, size_t(batch) * 3 * sizeof(float)),
+            buffer(d_->train_w, size_t(batch) * sizeof(float)),
+            buffer(d_->train_parts, (rows + 255) / 256 * sizeof(float)),
+        }));
         clear_graphs();
         SPB_RCUDA(cudaError_t(d_->net.prepare_gradients(batch)));
+        d_->train_capacity = batch;
     }
     if (!d_->pass_counter) {
         SPB_RCUDA(dev_malloc(&d_->pass_counter, sizeof(uint32_t)));
