@@ -119,6 +119,46 @@ def test_guided_cornell_matches_reference_image(case):
     assert worst < 0.02, f"worst 8x8 block deviation {worst:.4f}"
 
 
+@pytest.mark.parametrize("case", ["cornell64_lights", "builtins96"])
+def test_guided_split_selection_matches_reference_image(case):
+    """Guiding with every light-tree node above the split depth split: guided frames have a body of
+    their own for the selected lights' samples (picks, and the environment in the second slot), held
+    here to the reference's image as the plain one is by test_split_light_selection_matches_reference."""
+    import ctypes
+    import json
+    import pathlib
+
+    from sprout_b200 import _lib, capi, scenes
+
+    data = np.load(pathlib.Path(__file__).resolve().parent / "golden" / "cornell_reference.npz")
+    meta = json.loads(bytes(data["meta"]).decode())["cases"][case]
+    ref = data[case].astype(np.float64)
+    w, h = meta["width"], meta["height"]
+    su = capi.SuLibrary()
+    assert su.su_init(False) == 0
+    try:
+        scene = dict(meta["scene"])
+        build = scenes.builtin_shapes if scene.pop("scene", None) == "builtins" else scenes.cornell
+        integrator = {"guiding": True, "light_sampling": {"strategy": "Adaptive", "splitting_threshold": 1.0}}
+        build(su, w, h, spp=4 * meta["spp"], integrator=integrator, **scene)
+        if build is scenes.cornell:
+            su.su_create_defaults()
+        assert su.su_render_frame(0) == 0, su.messages
+        assert su.su_postprocess() == 0
+        img = su.framebuffer(w, h)[0][:, :, :3].astype(np.float64)
+        st = _lib.RenderStats()
+        assert _lib.load().spb_render_last_stats(ctypes.byref(st)) == 0
+        assert st.guide_vertices > 0
+    finally:
+        su.su_release()
+    m_ref, m_img = ref.mean(axis=(0, 1)), img.mean(axis=(0, 1))
+    assert np.all(np.abs(m_img - m_ref) <= 0.005 * m_ref), (m_img, m_ref)
+    b = meta.get("block", 8)
+    bi, br = block_means(img, b), block_means(ref, b)
+    worst = np.max(np.abs(bi - br) / (np.abs(br) + 0.01))
+    assert worst < 0.02, f"worst {b}x{b} block deviation {worst:.4f}"
+
+
 def test_guiding_settings_are_parsed():
     """The integrator's "guiding" object: explicit settings render, and training can stop
     early (train_spp) with the rest of the frame sampled by the frozen network."""

@@ -97,3 +97,22 @@ def test_forced_instancing_volume_matches_the_reference():
                      w, h)
     assert st["instances"] > 0 and st["tracking_capped"] == 0
     assert_close(img, ref, meta["block"])
+
+
+@pytest.mark.parametrize("instancing", [False, True], ids=["flat", "instanced"])
+@pytest.mark.parametrize("case", ["cornell64_grid", "volume64"])
+def test_split_selection_through_media_matches_the_reference(case, instancing):
+    """Picks of split light selections through a density grid, in both kinds of tree: the two triangles
+    of the Cornell lamp, and the many of the volume's sphere light beside its environment."""
+    ref, meta = golden(case)
+    w, h, spp = meta["width"], meta["height"], meta["spp"]
+    density = np.load(GOLDEN)[meta["density"]]
+    ptmis = {"instancing": instancing, "light_sampling": {"strategy": "Adaptive", "splitting_threshold": 1.0}}
+    if case == "volume64":
+        img, st = render(lambda su: scenes.volume(su, w, h, spp, density, integrator=ptmis), w, h)
+    else:
+        img, st = render(lambda su: scenes.cornell(su, w, h, tonemap=True, spp=spp, density=density, integrator=ptmis,
+                                                   **meta["scene"]), w, h)
+    assert (st["instances"] > 0) == instancing and st["overflow"] == 0 and st["tracking_capped"] == 0
+    assert np.all(np.isfinite(img))
+    assert_close(img, ref, meta.get("block", 8))
