@@ -61,7 +61,7 @@ typedef struct spb_tree_info {
     uint32_t num_nodes;       /* 8-wide nodes (96 bytes each) */
     uint32_t num_leaves;      /* leaf slots (1-3 triangles each) */
     uint32_t max_depth;       /* deepest node, root = 1 */
-    uint64_t device_bytes;    /* nodes + triangles resident on the device */
+    uint64_t device_bytes;    /* nodes + triangles (64 bytes each) resident on the device */
     double   build_seconds;   /* host build + upload time of the last build */
     double   sah_cost;        /* SAH cost of the 8-wide tree (traversal 1, triangle 1) */
 } spb_tree_info;
@@ -120,7 +120,8 @@ SPB_API int32_t spb_intersect_p_host(spb_tree* tree, float const* rays, uint64_t
  * Closest hit (device pointers, as spb_intersect_device) that also counts the traversal's
  * work: node_steps receives the 8-wide nodes visited and triangle_steps the triangles tested,
  * summed over all rays of the batch.  Synchronizes the stream before returning the counts.
- * For measurement (bytes fetched per ray: nodes x 96 + triangles x 48); the counting costs
+ * For measurement (bytes fetched per ray: nodes x 96 + triangles x 48, of the 64 bytes a
+ * triangle takes on the device); the counting costs
  * a few percent, so timed casts use spb_intersect_device.  The reference counts nothing of
  * the kind; its Tree::intersect (source/core/scene/shape/triangle/bvh/triangle_bvh_tree.cpp:41-90)
  * visits nodes and tests triangles in the same sense.

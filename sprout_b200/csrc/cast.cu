@@ -15,12 +15,15 @@
 //  * Traversal, triangle test and hit definition: traverse.cuh.
 //
 // What bounds it, and what it measured (B200; before: every lane stepping by itself through
-// 80-byte nodes, one launch form): the start's kernel kept 9.8 of 32 lanes busy and its ALU pipe
-// 70 % (29 warp instructions a step); now 19.4 lanes and 12, and what is left is the latency of
-// dependent node loads (32 warps an SM) and L1's one tag look-up a cycle for each lane's line.
-//   16,777,216 incoherent closest-hit rays, 1,048,576 triangles: 2,540 -> 1,205 us
-//   4,194,301 short any-hit rays from its surface: 2,600 -> 1,265 us
-//   360,000 primary rays, 65,536 triangles: 253 -> 125 us; 4,099 any-hit rays: 37 -> 23 us
+// 80-byte nodes, one launch form).  On 4,194,301 short any-hit rays from the surface of 1,048,576
+// triangles 9.8 of 32 lanes were busy and the ALU pipe 70 % (29 warp instructions a step); together
+// 18.9 lanes are, the ALU pipe is at 51 %, and what is left is the latency of dependent node loads
+// (5.8 stalls an instruction, 31 warps an SM) and L1's one tag look-up a cycle for each lane's line
+// (62 % of its rate).  Casts one after another on a stream, us:
+//   16,777,216 incoherent closest-hit rays, 1,048,576 triangles: 2,540 -> 1,205
+//   those 4,194,301 any-hit rays: 2,600 -> 1,265 (1,300 with a wait after each)
+//   360,000 primary rays, 65,536 triangles: 253 -> 125
+//   4,099 any-hit rays: 37 -> 23 (38 -> 27 with a wait after each)
 // Tried and not kept: ray batches copied to shared memory ahead of use (cp.async, one batch ahead:
 // 1,250, 1,360 and 170 us on the first three, for claimed batches wait while other warps run dry);
 // the closest hit's barycentrics recomputed at the end instead of carried (1 % slower).
@@ -90,9 +93,12 @@ __device__ __forceinline__ void answer_miss(uint32_t i, float t, uint32_t* ids, 
 }
 
 // Chooses the form of a large cast: *sparse = 1 if most of Probes rays spread over the batch miss
-// the scene box.  One block of Probes threads.  (The sparse form: 16,777,216 rays of which 28 %
-// enter, 1,205 against 1,566 us; 4,194,301 rays that all enter, 1,320 against 1,265 us, because
-// its queue takes registers from the walk.)
+// the scene box.  One block of Probes threads.  The sparse form against the dense one, closest hits
+// of incoherent rays around 1,048,576 triangles, us at 2^20 / 2^24 rays: 28 % entering 215 / 1,216
+// against 232 / 1,617, half 240 / 1,932 against 252 / 2,267, three quarters 275 / 2,822 against
+// 274 / 3,009, all 380 / 4,156 against 354 / 4,158 (its queue takes registers from the walk; 4,194,301
+// any-hit rays that all enter: 1,320 against 1,265).  Half is thus on the safe side of the line at
+// every size.
 __global__ void choose_kernel(float4 const* __restrict__ rays, uint32_t num_rays, float3 scene_lo, float3 scene_hi,
                               uint32_t* __restrict__ sparse) {
     uint32_t const i = uint32_t(uint64_t(threadIdx.x) * num_rays / Probes);

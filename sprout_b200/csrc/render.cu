@@ -2215,7 +2215,8 @@ SPB_HD bool grid_tracked(shading::Material const& m) { return m.medium != 0 && !
 // (Tracking_multi::integrate heterogeneous branch, tracking_multi.cpp:98-164, with
 // Tracking::tracking over a majorant cell, tracking.cpp:286-349); emitting grids are tracked by
 // k_shade.  p.track receives the path weight and the distance of a scattering event (below zero:
-// none), p.rng the random numbers' state.  Persistent warps, a path a lane (see k_transmit).
+// none), p.rng the random numbers' state.  Persistent warps, a path a lane (see k_transmit; 16.8
+// lanes, 50 % of the issue slots).
 __global__ void __launch_bounds__(Trace_block, 5)
     k_track(__grid_constant__ Scene_gpu const s, Paths p, uint32_t const* __restrict__ queue,
             uint32_t const* __restrict__ count, uint32_t* fetch) {
@@ -2337,11 +2338,13 @@ __global__ void __launch_bounds__(Trace_block, 5)
 // ---- shade: one path vertex ----
 // Media: the scene has participating media.  Guided: path guiding.  Textured: some material has
 // maps.  A frame takes the variant without what it does not use (shade_kernel), and next_event has
-// one body for every light: the kernel waits on instruction fetch (4.0 of its 10 stalls an
-// instruction; 16.5 of 32 lanes, 2,700 instructions a warp, each fetched about once), so what
-// counts is the code a warp runs through.  512 x 512 x 64 Cornell frame 25.4 -> 23.3 ms, 960 x 540
-// x 32 instanced frame 85.5 -> 82.0 ms.  Blocks of 128 threads with registers for 5, 6 or 8 of them
-// on an SM (96, 80, 64) spill and are no faster.
+// one body for every light: with all in one kernel it waited on instruction fetch (4.0 of its 10
+// stalls an instruction; 16.5 of 32 lanes, 2,700 instructions a warp, each fetched about once), so
+// what counts is the code a warp runs through.  512 x 512 x 64 Cornell frame 25.4 -> 23.3 ms, 960 x
+// 540 x 32 instanced frame 85.5 -> 82.0 ms.  The variant of the Cornell box now stalls 2.4 on loads,
+// 2.4 on fixed latencies and 0.4 (first vertex) to 2.0 (later ones) on instruction fetch, at 15 warps
+// an SM (127 registers).  Blocks of 128 threads with registers for 5, 6 or 8 of them on an SM (96,
+// 80, 64) spill and are no faster.
 template <bool Media, bool Guided, bool Textured>
 __global__ void __launch_bounds__(Shade_block)
     k_shade(__grid_constant__ Scene_gpu const s, Launch const* __restrict__ launch, Paths p, uint32_t const* __restrict__ q_in,
@@ -2741,7 +2744,9 @@ Shade_kernel shade_kernel(bool media, bool guided, bool textured) {
 // walk on (cell_step) until Walk_threshold of them are through.  (One thread a ray from start to
 // end kept 7.9 of 32 lanes busy.)  Boundaries are looked for in a tree of their own: in the scene's
 // tree a ray to a lamp walks through all of the lamp's triangles.  What is left: 130 to 200
-// instructions a cell (64-bit random numbers, a logarithm, face distances) at about half the lanes.
+// instructions a cell (64-bit random numbers, a logarithm, face distances) at half the lanes (16.3),
+// 53 % of the issue slots at 19 warps an SM (96 registers), load latency the first of its stalls (3.6
+// an instruction).
 // Three 384 x 384 x 32 views of a 256^3 grid, whole frame: 106.5 ms before; 85.5 with this kernel
 // and k_track, 74.0 with the boundary tree and registers for 5 blocks an SM.
 //
@@ -3019,7 +3024,6 @@ __device__ __forceinline__ float filter_weight(Filter_table const& f, float d) {
 
 // Bound by the loads of the nine samples around each film pixel, mostly L1 hits.  A wave of
 // 256 x 256 x 31 samples: 167 us with the table in constant memory, 88 us.
-
 __global__ void k_gather(Paths p, Launch const* __restrict__ launch, uint32_t film_pixels, uint32_t samples,
                          float4* film, float4* comp) {
     __shared__ Filter_table filter;
@@ -3207,7 +3211,7 @@ __device__ bool spec_track_homogeneous(spec::V4 mu_a, spec::V4 mu_s, float t, fl
     return false;
 }
 
-// Delta tracking with spectral MIS through a density grid (track_grid over the carried
+// Delta tracking with spectral MIS through a density grid (as k_track, over the carried
 // wavelengths); maj_t bounds the coefficients at density 1 for every wavelength.
 __device__ __forceinline__ bool spec_track_grid(bool on, Medium_gpu const& g, float maj_t, spec::V4 mu_a, spec::V4 mu_s, V3 ro, V3 rd,
                                 float t0, float t1, Rng& rng, float& t_out, spec::V4& lw, uint32_t* capped) {
@@ -3268,7 +3272,7 @@ __device__ __forceinline__ bool spec_track_grid(bool on, Medium_gpu const& g, fl
     return scattered;
 }
 
-// Ratio tracking through a density grid (transmit_grid over the carried wavelengths): w is
+// Ratio tracking through a density grid (as k_transmit, over the carried wavelengths): w is
 // multiplied by the estimate; false when it falls below Abort_epsilon.
 __device__ __forceinline__ bool spec_transmit_grid(bool on, Medium_gpu const& g, float maj_t, float min_t, spec::V4 mu_t, V3 ro, V3 rd,
                                    float t0, float t1, Rng& rng, spec::V4& w, uint32_t* capped) {
@@ -3490,9 +3494,9 @@ constexpr int Spectral_plain = 0, Spectral_train = 1, Spectral_guided = 2;
 // traversal, tracking, the scattering vertex, its shadow ray's walk, the continuation.  Lanes whose
 // path has ended splat it and take new ones once Regenerate_threshold of them have.  (A thread a
 // path, from start to end, kept 3.9 of 32 lanes busy.)  Two 256 x 256 x 24 views of a 256^3 grid:
-// 57.4 -> 42.6 ms.  What is left: instruction fetch (6.6 of its stalls an instruction), and lanes
-// that wait for the longest walk of their warp.  Registers for 3 or 5 blocks an SM: 6 and 3 %
-// slower.
+// 57.4 -> 42.6 ms.  What is left: instruction fetch (on a 64^3 grid 13.5 stalls an instruction, before
+// 17.0), and lanes that wait for the longest walk of their warp (9.3 of 32 busy there, before 4.4).
+// Registers for 3 or 5 blocks an SM: 6 and 3 % slower.
 constexpr int Regenerate_threshold = 8;
 
 template <int Mode>

@@ -4,7 +4,8 @@
 // Traversal follows the compressed-wide-BVH scheme of Ylitie, Karras and Laine (HPG 2017):
 // a node group (child base, hit bits) and a triangle group (triangle base, hit bits) per
 // lane, a per-lane stack of pending node groups, children visited in the ray-octant order
-// fixed at build time.  One step is one node (8 child boxes) or one triangle.
+// fixed at build time.  A warp steps together (warp_step): each lane tests one pending triangle,
+// if it has any, then, if none is left, the next node (8 child boxes).
 //
 // The triangle test is the reference's Möller-Trumbore (triangle_primitive_mt.inl:100-131)
 // with its operation order: cross products as in simd.inl:173-187 (AVX2 path: one product
