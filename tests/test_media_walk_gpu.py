@@ -125,15 +125,12 @@ def test_coloured_constant_grid_in_waves_smaller_than_a_warp(side):
     _assert_same_mean(*means)
 
 
-@pytest.mark.parametrize("instancing", [False, True], ids=["flat", "instanced"])
-@pytest.mark.parametrize("spectral", [False, True], ids=["rgb", "spectral"])
-def test_absorbing_grid_has_the_closed_form_transmittance(spectral, instancing):
+@pytest.mark.parametrize("mode", ["rgb", "instanced", "spectral"])
+def test_absorbing_grid_has_the_closed_form_transmittance(mode):
     """Density that varies from voxel to voxel, absorption only: what the camera sees through the grid
     is the environment times exp(-mu_t x the density along the ray), which numpy integrates.  The
     density is a product of a tent along each axis, so that the trilinear filter interpolates each tent
     linearly and wrapping or clamping at the border are the same."""
-    if spectral and instancing:
-        pytest.skip("the spectral mode takes flat scenes")
     n, side, spp, mu_t, sky = 21, 33, 512, 1.5, 0.4
     centre = (np.arange(n) + 0.5) / n
     tent = 1.0 - np.abs(2.0 * centre - 1.0)
@@ -141,8 +138,8 @@ def test_absorbing_grid_has_the_closed_form_transmittance(spectral, instancing):
     medium = {"attenuation_color": [0.5] * 3, "attenuation_distance": float(np.log(2.0) / mu_t),
               "subsurface_color": [0.0] * 3, "anisotropy": 0.0}
     position = (0.25, 0.15, -1.9)  # the cube fills the view, the lamp is behind the camera's shoulder
-    got, _ = _channel_means(side, spp, density, {"spectral": spectral, "instancing": instancing}, medium=medium,
-                            position=position, environment=(sky, sky, sky))
+    got, _ = _channel_means(side, spp, density, MODES[mode], medium=medium, position=position,
+                            environment=(sky, sky, sky))
     # rays through 3 x 3 points of each pixel
     m = scenes._look_at(position).astype(np.float64)
     at = (np.arange(3 * side) + 0.5) / (3 * side) * 2.0 - 1.0
